@@ -146,6 +146,12 @@ PT_API pt_status pt_set_bvh_builder(pt_context *ctx, uint32_t builder);
  * leaf-ordered records are copied out. */
 PT_API pt_status pt_debug_build_bvh(const float *positions, uint32_t triangles, uint32_t spatial, double stats[6],
                                     void *nodes, uint64_t node_capacity, void *records, uint64_t record_capacity);
+/* Host-only: the 64-byte four-child node over four child boxes (lo / hi by
+ * axis, then child) with child references `ref` (-1: unused slot), as the
+ * builders write it: base x y z, step x | step y, step z, lower x planes,
+ * upper x planes | lower y, upper y, lower z, upper z | references. Plane
+ * byte q of child i lies at base + step * (1 + q / 32768). */
+PT_API pt_status pt_debug_pack_node4(const float lo[12], const float hi[12], const int32_t ref[4], uint32_t out[16]);
 /* 1 when the scene's current BVH was built on the device. */
 PT_API pt_status pt_scene_bvh_on_device(pt_context *ctx, uint32_t scene_id, int *on_device);
 /* Host wall time in seconds of the scene's pt_scene_upload: [0] the host

@@ -1,0 +1,101 @@
+// The quantised four-child node (Bvh4Node): how the builders and the refit
+// write one, on the host and on the device.
+#pragma once
+
+#include <cmath>
+#include <cstdint>
+#include <cstring>
+
+#include <vector_functions.h>
+
+#include "dev_types.h"
+
+#ifdef __CUDACC__
+#define PT_HD __host__ __device__ __forceinline__
+#else
+#define PT_HD inline
+#endif
+
+namespace ptd {
+
+// Fills `out` from the boxes of up to four children (lo[axis][child],
+// hi[axis][child]; used for refs other than kEmptyChild). Every stored plane
+// lies on or outside the box it stands for: the lower ones are rounded down
+// and the upper ones up, in f64, against the plane positions the node
+// decodes to. An axis whose extent has no finite grid (infinite or huge
+// coordinates, every child's box empty) decodes to NaN planes, which bound
+// nothing; a child whose own box is empty (NaN corners) spans the node's.
+PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4], Bvh4Node &out) {
+  float base[3], step[3];
+  uint32_t qlo[3], qhi[3];
+  for (int a = 0; a < 3; ++a) {
+    float l = INFINITY, h = -INFINITY;
+    for (int i = 0; i < 4; ++i)
+      if (ref[i] != kEmptyChild) {
+        l = fminf(l, lo[a][i]);
+        h = fmaxf(h, hi[a][i]);
+      }
+    int e = 0;
+    const double range = (double)h - (double)l;
+    bool grid = range >= 0.0 && range < 1.0e38;
+    if (grid) {
+      frexp(range / 253.0, &e);
+      // Not finer than the coordinates can resolve: the f64 sums below stay
+      // exact, and a box without extent gets a grid all the same.
+      int least = -100;
+      const double most = fmax(fabs((double)l), fabs((double)h));
+      if (most > 0.0) {
+        frexp(most, &least);
+        least = least - 30 < -100 ? -100 : least - 30;
+      }
+      e = range == 0.0 || e < least ? least : e;
+    }
+    double s = 1.0, origin = 0.0;
+    for (; grid; ++e) {
+      s = ldexp(1.0, e);
+      const double wide = s * 32768.0;
+      if (!(wide < 1.0e38)) {
+        grid = false;
+        break;
+      }
+      const double want = (double)l - wide;
+      float b = (float)want;
+      if ((double)b > want) b = nextafterf(b, -INFINITY);
+      if (!(fabsf(b) < 1.0e38f)) {
+        grid = false;
+        break;
+      }
+      origin = (double)b + wide;
+      base[a] = b;
+      step[a] = (float)wide;
+      if (ceil(((double)h - origin) / s) <= 255.0) break;
+    }
+    qlo[a] = 0u;
+    qhi[a] = 0u;
+    if (!grid) {
+      base[a] = -INFINITY;
+      step[a] = INFINITY;
+    }
+    for (int i = 0; i < 4; ++i) {
+      uint32_t l8 = 255u, h8 = 0u;
+      if (ref[i] != kEmptyChild) {
+        l8 = 0u;
+        h8 = 255u;
+        if (grid && lo[a][i] <= hi[a][i]) {
+          l8 = (uint32_t)fmax(floor(((double)lo[a][i] - origin) / s), 0.0);
+          h8 = (uint32_t)ceil(((double)hi[a][i] - origin) / s);
+        }
+      }
+      qlo[a] |= l8 << (8 * i);
+      qhi[a] |= h8 << (8 * i);
+    }
+  }
+  out.base = make_float4(base[0], base[1], base[2], step[0]);
+  out.mid = make_uint4(0, 0, qlo[0], qhi[0]);
+  memcpy(&out.mid.x, &step[1], 4);
+  memcpy(&out.mid.y, &step[2], 4);
+  out.planes = make_uint4(qlo[1], qhi[1], qlo[2], qhi[2]);
+  out.child = make_int4(ref[0], ref[1], ref[2], ref[3]);
+}
+
+}  // namespace ptd

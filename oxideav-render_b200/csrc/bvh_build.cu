@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "bvh_build.h"
+#include "bvh4.h"
 #include "dev_types.h"
 
 namespace ptd {
@@ -569,14 +570,7 @@ __global__ void k_write_nodes(Nodes nd, const uint64_t *offs, BvhNode *out2, Bvh
         }
       }
       Bvh4Node q;
-      q.lo_x = make_float4(bl[0][0], bl[0][1], bl[0][2], bl[0][3]);
-      q.hi_x = make_float4(bh[0][0], bh[0][1], bh[0][2], bh[0][3]);
-      q.lo_y = make_float4(bl[1][0], bl[1][1], bl[1][2], bl[1][3]);
-      q.hi_y = make_float4(bh[1][0], bh[1][1], bh[1][2], bh[1][3]);
-      q.lo_z = make_float4(bl[2][0], bl[2][1], bl[2][2], bl[2][3]);
-      q.hi_z = make_float4(bh[2][0], bh[2][1], bh[2][2], bh[2][3]);
-      q.child = make_int4(ref[0], ref[1], ref[2], ref[3]);
-      q.pad = make_int4(0, 0, 0, 0);
+      pack_bvh4(bl, bh, ref, q);
       out4[(uint32_t)o] = q;
     }
   }
@@ -1031,14 +1025,7 @@ __global__ void k_sah_write_nodes(SahNodes nd, uint32_t total, const uint64_t *o
       }
     }
     Bvh4Node q;
-    q.lo_x = make_float4(bl[0][0], bl[0][1], bl[0][2], bl[0][3]);
-    q.hi_x = make_float4(bh[0][0], bh[0][1], bh[0][2], bh[0][3]);
-    q.lo_y = make_float4(bl[1][0], bl[1][1], bl[1][2], bl[1][3]);
-    q.hi_y = make_float4(bh[1][0], bh[1][1], bh[1][2], bh[1][3]);
-    q.lo_z = make_float4(bl[2][0], bl[2][1], bl[2][2], bl[2][3]);
-    q.hi_z = make_float4(bh[2][0], bh[2][1], bh[2][2], bh[2][3]);
-    q.child = make_int4(ref[0], ref[1], ref[2], ref[3]);
-    q.pad = make_int4(0, 0, 0, 0);
+    pack_bvh4(bl, bh, ref, q);
     out4[(uint32_t)o] = q;
   }
 }

@@ -16,6 +16,7 @@
 
 #include <string>
 
+#include "bvh4.h"
 #include "dev_scene.cuh"
 #include "host_scene.h"
 
@@ -155,7 +156,7 @@ __global__ void k_refit4_links(const Bvh4Node *nodes, uint32_t n, uint32_t *pare
     const int ch[4] = {nodes[i].child.x, nodes[i].child.y, nodes[i].child.z, nodes[i].child.w};
     uint32_t c = 0;
     for (int k = 0; k < 4; ++k)
-      if (ch[k] >= 0 && ch[k] != kEmptyChild && (uint32_t)ch[k] < n) {
+      if (ch[k] >= 0 && (uint32_t)ch[k] < n) {
         parent[ch[k]] = i;
         ++c;
       }
@@ -163,79 +164,61 @@ __global__ void k_refit4_links(const Bvh4Node *nodes, uint32_t n, uint32_t *pare
   }
 }
 
-__device__ __forceinline__ float lane(const float4 &v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); }
-__device__ __forceinline__ void set_lane(float4 &v, int k, float x) {
-  if (k == 0)
-    v.x = x;
-  else if (k == 1)
-    v.y = x;
-  else if (k == 2)
-    v.z = x;
-  else
-    v.w = x;
-}
-
+// `boxes`: the bounds of each finished node's subtree (lo, hi), which its
+// parent reads; the nodes themselves hold them quantised.
 __global__ void k_refit4_up(Bvh4Node *nodes, uint32_t n, const float4 *records, const uint32_t *parent,
-                            uint32_t *pending) {
+                            uint32_t *pending, float4 *boxes) {
   for (uint32_t start = blockIdx.x * blockDim.x + threadIdx.x; start < n; start += gridDim.x * blockDim.x) {
     bool interior = false;
     {
       const int4 c = nodes[start].child;
       const int ch[4] = {c.x, c.y, c.z, c.w};
-      for (int k = 0; k < 4; ++k) interior |= ch[k] >= 0 && ch[k] != kEmptyChild && (uint32_t)ch[k] < n;
+      for (int k = 0; k < 4; ++k) interior |= ch[k] >= 0 && (uint32_t)ch[k] < n;
     }
     if (interior) continue;
     uint32_t i = start;
     for (;;) {
-      Bvh4Node nd = nodes[i];
-      const int ch[4] = {nd.child.x, nd.child.y, nd.child.z, nd.child.w};
+      const int4 c = nodes[i].child;
+      const int ch[4] = {c.x, c.y, c.z, c.w};
+      float bl[3][4], bh[3][4];
+      float4 ulo = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+      float4 uhi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
       for (int k = 0; k < 4; ++k) {
-        float lo[3], hi[3];
-        bool ok = false;
-        if (ch[k] == kEmptyChild) continue;
-        if (ch[k] < 0) {
-          ok = leaf_bounds(records, ch[k], lo, hi);
-        } else if ((uint32_t)ch[k] < n) {
-          const Bvh4Node *c = nodes + ch[k];
-          const float4 lx = __ldcg(&c->lo_x), hx = __ldcg(&c->hi_x), ly = __ldcg(&c->lo_y), hy = __ldcg(&c->hi_y);
-          const float4 lz = __ldcg(&c->lo_z), hz = __ldcg(&c->hi_z);
-          const int4 cc = __ldcg(&c->child);
-          const int gch[4] = {cc.x, cc.y, cc.z, cc.w};
-          for (int a = 0; a < 3; ++a) {
-            lo[a] = INFINITY;
-            hi[a] = -INFINITY;
+        float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        if (ch[k] != kEmptyChild) {
+          if (ch[k] < 0) {
+            leaf_bounds(records, ch[k], lo, hi);
+          } else if ((uint32_t)ch[k] < n) {
+            const float4 l = __ldcg(boxes + 2 * (size_t)ch[k]), h = __ldcg(boxes + 2 * (size_t)ch[k] + 1);
+            lo[0] = l.x;
+            lo[1] = l.y;
+            lo[2] = l.z;
+            hi[0] = h.x;
+            hi[1] = h.y;
+            hi[2] = h.z;
           }
-          for (int j = 0; j < 4; ++j) {
-            if (gch[j] == kEmptyChild) continue;
-            lo[0] = fminf(lo[0], lane(lx, j));
-            hi[0] = fmaxf(hi[0], lane(hx, j));
-            lo[1] = fminf(lo[1], lane(ly, j));
-            hi[1] = fmaxf(hi[1], lane(hy, j));
-            lo[2] = fminf(lo[2], lane(lz, j));
-            hi[2] = fmaxf(hi[2], lane(hz, j));
-            ok = true;
-          }
+          ulo = make_float4(fminf(ulo.x, lo[0]), fminf(ulo.y, lo[1]), fminf(ulo.z, lo[2]), 0.0f);
+          uhi = make_float4(fmaxf(uhi.x, hi[0]), fmaxf(uhi.y, hi[1]), fmaxf(uhi.z, hi[2]), 0.0f);
         }
-        if (!ok) continue;
         float plo[3], phi[3];
         pad_bounds(lo, hi, plo, phi);
-        set_lane(nd.lo_x, k, plo[0]);
-        set_lane(nd.hi_x, k, phi[0]);
-        set_lane(nd.lo_y, k, plo[1]);
-        set_lane(nd.hi_y, k, phi[1]);
-        set_lane(nd.lo_z, k, plo[2]);
-        set_lane(nd.hi_z, k, phi[2]);
+        for (int a = 0; a < 3; ++a) {
+          bl[a][k] = plo[a];
+          bh[a][k] = phi[a];
+        }
       }
-      nodes[i].lo_x = nd.lo_x;
-      nodes[i].hi_x = nd.hi_x;
-      nodes[i].lo_y = nd.lo_y;
-      nodes[i].hi_y = nd.hi_y;
-      nodes[i].lo_z = nd.lo_z;
-      nodes[i].hi_z = nd.hi_z;
+      Bvh4Node nd;
+      pack_bvh4(bl, bh, ch, nd);
+      nodes[i].base = nd.base;
+      nodes[i].mid = nd.mid;
+      nodes[i].planes = nd.planes;
+      boxes[2 * (size_t)i] = ulo;
+      boxes[2 * (size_t)i + 1] = uhi;
       __threadfence();
       const uint32_t p = parent[i];
       if (p == kNoParent) break;
       if (atomicSub(&pending[p], 1u) != 1u) break;
+      __threadfence();
       i = p;
     }
   }
@@ -257,12 +240,15 @@ std::string device_refit_bvh(SceneHost &sc, uint64_t records, cudaStream_t st) {
   const uint32_t n2 = d.node_count, n4 = d.node4_count;
   const uint64_t nmax = std::max<uint64_t>(std::max(n2, n4), 1);
   uint32_t *scratch = nullptr;
-  cudaError_t e = cudaMallocAsync((void **)&scratch, 2 * nmax * sizeof(uint32_t), st);
+  // Links and counts of either layout, then the four-child nodes' bounds.
+  const uint64_t links = (2 * nmax * sizeof(uint32_t) + 255) & ~uint64_t(255);
+  cudaError_t e = cudaMallocAsync((void **)&scratch, links + 2 * (uint64_t)n4 * sizeof(float4), st);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return std::string("refit scratch: ") + cudaGetErrorString(e);
   }
   uint32_t *parent = scratch, *pending = scratch + nmax;
+  float4 *boxes = reinterpret_cast<float4 *>(reinterpret_cast<uint8_t *>(scratch) + links);
   if (n2) {
     e = cudaMemsetAsync(parent, 0xff, n2 * sizeof(uint32_t), st);
     k_refit2_links<<<grid_of(n2), kRefitThreads, 0, st>>>(d.nodes, n2, parent, pending);
@@ -272,7 +258,7 @@ std::string device_refit_bvh(SceneHost &sc, uint64_t records, cudaStream_t st) {
     e = cudaMemsetAsync(parent, 0xff, n4 * sizeof(uint32_t), st);
     k_refit4_links<<<grid_of(n4), kRefitThreads, 0, st>>>(d.nodes4, n4, parent, pending);
     k_refit4_up<<<grid_of(n4), kRefitThreads, 0, st>>>(const_cast<Bvh4Node *>(d.nodes4), n4, d.tris, parent,
-                                                        pending);
+                                                        pending, boxes);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
   cudaFreeAsync(scratch, st);

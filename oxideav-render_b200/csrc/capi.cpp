@@ -18,6 +18,7 @@
 
 #include "../../include/pt_b200.h"
 #include "../../include/pt_b200_debug.h"
+#include "bvh4.h"
 #include "context.h"
 #include "host_scene.h"
 #include "kernels.h"
@@ -1324,6 +1325,18 @@ pt_status pt_debug_build_bvh(const float *positions, uint32_t triangles, uint32_
     if (records && record_capacity >= rec.size() / 3) std::memcpy(records, rec.data(), rec.size() * sizeof(float4));
     return PT_OK;
   });
+}
+
+pt_status pt_debug_pack_node4(const float lo[12], const float hi[12], const int32_t ref[4], uint32_t out[16]) {
+  if (!lo || !hi || !ref || !out) return fail(nullptr, PT_ERR_INVALID_ARG, "NULL argument");
+  float l[3][4], h[3][4];
+  std::memcpy(l, lo, sizeof l);
+  std::memcpy(h, hi, sizeof h);
+  Bvh4Node n;
+  pack_bvh4(l, h, ref, n);
+  static_assert(sizeof n == 64, "four-child nodes are 64 bytes");
+  std::memcpy(out, &n, sizeof n);
+  return PT_OK;
 }
 
 pt_status pt_autotune(pt_context *ctx, pt_tracer *t, uint32_t samples, pt_tune_choice *best) {

@@ -1,19 +1,23 @@
 // Persistent-thread traversal for the wavefront's extend and shadow kernels.
 //
-// Each lane owns one ray at a time and asks for the next queue entry the
-// moment its ray finishes (one warp-aggregated atomic per refill), so the
-// lanes of a warp stay busy instead of idling behind the warp's slowest ray
-// (Aila & Laine, "Understanding the Efficiency of Ray Traversal on GPUs",
-// HPG 2009: persistent threads with dynamic fetch) and the warp alternates a
-// speculative node phase with a leaf phase (their while-while traversal
-// with postponed leaves), so lanes rarely idle behind each other; the node
-// phase does not wait for its last few searching lanes
-// (node_phase_goes_on).
+// Each lane owns one ray at a time; a warp takes new rays from the queue
+// when enough of its lanes stand idle (Aila & Laine, "Understanding the
+// Efficiency of Ray Traversal on GPUs", HPG 2009: persistent threads with
+// dynamic fetch). A ray has up to two pieces of work at hand: a node to
+// visit and triangles of one parked leaf to test (their speculative
+// traversal with postponed leaves). Each step the warp votes which kind of
+// work to do, one node visit or one triangle test per lane that has it, so
+// whichever more lanes wait for goes first and no phase is held up by its
+// slowest lane.
 //
-// The traversal stack keeps its top entries in shared memory (one column
-// per thread, conflict-free) and spills deeper entries to local memory.
-// Rays walk either node layout of the scene: two-child 64-byte nodes or the
-// same tree as four-child 128-byte nodes (fewer, wider steps).
+// The traversal stack keeps its first entries in shared memory (one column
+// per thread, conflict-free) and the deeper ones in local memory. Rays walk
+// either node layout of the scene: two-child 64-byte nodes or the same tree
+// as quantised four-child 64-byte nodes (fewer, wider steps).
+//
+// These loops are bound by instruction issue and by the registers that a
+// resident ray takes (1,024 rays an SM leave 64 each), so what a ray can
+// look up again when it needs it, at a hit or at its end, is not held.
 //
 // Results equal closest_hit / occluded of dev_scene.cuh: the closest hit is
 // the accepted candidate with the smallest t (ties: lowest global id), a
@@ -25,326 +29,316 @@
 
 namespace ptd {
 
-// Shared-memory entries per thread. Eight keep the blocks' shared memory
-// small, which leaves more of the SM's L1 to node and triangle data; the
-// request mix traced 1 % faster than with 16 (24: no change).
-constexpr int kShortStack = 8;
-constexpr int kTravDone = kEmptyChild;  // "no next node" (never a node index)
+// Stack entries a thread keeps in shared memory. A node visit whose pushes
+// stay within them takes the short, branch-free way; L1 loses what they take.
+// Extend + shadow stage at 8 / 12 / 16 / 20 / 24 entries: 500k-triangle soup
+// 109.7 / 103.5 / 95.9 / 94.1 / 93.5 ms a frame, stress scene 69.1 / 64.5 /
+// 62.9 / 64.0 / 63.6 ms, sphere grid 49.5 / 48.7 / 48.6 / 49.1 / 49.2 ms.
+constexpr int kShortStack = 16;
+constexpr int kTravDone = (int)0x80000000;  // "no next node": neither a node index nor a leaf reference
 // A four-child node pushes at most three entries per level and the builder
 // keeps the binary tree (hence the four-child tree) at most 56 levels deep.
 constexpr int kTravStackSize = 3 * 56 + 8;
+// Rows of a block's shared words, one word per thread each: the stack, then
+// the thread's node visits, triangle tests and rays.
+enum TravRows : int { ROW_NODES = kShortStack, ROW_TRIS, ROW_RAYS, ROW_COUNT };
 
+PT_DEV int shared_load(uint32_t a) {
+  int v;
+  asm volatile("ld.shared.s32 %0, [%1];" : "=r"(v) : "r"(a));
+  return v;
+}
+PT_DEV void shared_store(uint32_t a, int v) { asm volatile("st.shared.s32 [%0], %1;" ::"r"(a), "r"(v)); }
+
+// A thread's stack: `sp` is the shared byte address of the next free row of
+// its column (rows past kShortStack live in `spill`); kThreads is a power of
+// two, so the address gives the column too.
+template <int kThreads>
 struct TravStack {
-  int *sm;        // this thread's column: entry i at sm[i * stride]
-  int stride;
+  static constexpr uint32_t kRow = 4u * kThreads;
+  uint32_t sp;
   int spill[kTravStackSize - kShortStack];
-  PT_DEV void push(int &sp, int v, uint32_t &err) {
-    if (sp < kShortStack)
-      sm[sp * stride] = v;
-    else if (sp < kTravStackSize)
-      spill[sp - kShortStack] = v;
-    else {
-      err |= ERR_STACK_OVERFLOW;
-      return;
-    }
-    ++sp;
+  // The block's shared words start at address `words` (a constant).
+  static PT_DEV uint32_t limit(uint32_t words) { return words + kShortStack * kRow; }
+  // An empty stack holds kTravDone, so popping needs no test.
+  PT_DEV void reset(uint32_t words) {
+    sp = words + 4u * threadIdx.x;
+    shared_store(sp, kTravDone);
+    sp += kRow;
   }
-  // Callers pop only a non-empty stack; an empty one reads as "done".
-  PT_DEV int pop(int &sp) {
-    if (sp <= 0) return kTravDone;
-    --sp;
-    return sp < kShortStack ? sm[sp * stride] : spill[sp - kShortStack];
+  PT_DEV bool room_for_three(uint32_t words) const { return sp < limit(words) - 2u * kRow; }
+  PT_DEV void push_shared(bool yes, int v) {
+    if (yes) {
+      shared_store(sp, v);
+      sp += kRow;
+    }
+  }
+  PT_DEV int pop_shared() {
+    sp -= kRow;
+    return shared_load(sp);
+  }
+  PT_DEV void push(uint32_t words, int v, DevCounters *ctr) {
+    const uint32_t lim = limit(words);
+    if (sp < lim) {
+      shared_store(sp, v);
+    } else {
+      const uint32_t i = (sp - lim) / kRow;
+      if (i >= (uint32_t)(kTravStackSize - kShortStack)) {
+        atomicOr(&ctr->error_flags, (unsigned)ERR_STACK_OVERFLOW);
+        return;
+      }
+      spill[i] = v;
+    }
+    sp += kRow;
+  }
+  PT_DEV int pop(uint32_t words) {
+    const uint32_t lim = limit(words);
+    sp -= kRow;
+    return sp < lim ? shared_load(sp) : spill[(sp - lim) / kRow];
+  }
+  // One more of what `row` counts for this thread.
+  PT_DEV void count(uint32_t words, int row) const {
+    const uint32_t a = words + ((sp - words) & (kRow - 1u)) + (uint32_t)row * kRow;
+    asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(a));
   }
 };
 
-// Slab test of one child box against [t0, t1] (the test node_boxes applies).
-PT_DEV bool child_box(float lox, float hix, float loy, float hiy, float loz, float hiz, const Ray &r, float t0,
-                      float t1, float &entry) {
-  const float grow = 1.0000003576f;  // 1 + 2 * gamma(3)
-  float lx = (lox - r.o.x) * r.inv.x, hx = (hix - r.o.x) * r.inv.x;
-  float ly = (loy - r.o.y) * r.inv.y, hy = (hiy - r.o.y) * r.inv.y;
-  float lz = (loz - r.o.z) * r.inv.z, hz = (hiz - r.o.z) * r.inv.z;
-  float tn = fmaxf(fmaxf(fminf(lx, hx), fminf(ly, hy)), fmaxf(fminf(lz, hz), t0));
-  float tf = fminf(fminf(fmaxf(lx, hx), fmaxf(ly, hy)), fmaxf(lz, hz)) * grow;
-  tf = fminf(tf, t1);
-  entry = tn;
-  return tn <= tf;
+// One quantised plane of Bvh4Node: 1 + q / 32768 for byte i of `word`.
+PT_DEV float plane_at(uint32_t word, int i) {
+  return __uint_as_float(__byte_perm(word, 0x3f800000u, 0x7604u + ((uint32_t)i << 4)));
+}
+// The largest / smallest of three; NaN operands are passed over.
+PT_DEV float max3f(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+PT_DEV float min3f(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+PT_DEV int child_of(const int4 &c, uint32_t key) {
+  const int a = (key & 1u) ? c.y : c.x, b = (key & 1u) ? c.w : c.z;
+  return (key & 2u) ? b : a;
 }
 
-PT_DEV void cswap(float &ea, int &ca, float &eb, int &cb) {
-  if (eb < ea) {
-    float te = ea;
-    ea = eb;
-    eb = te;
-    int tc = ca;
-    ca = cb;
-    cb = tc;
+// Where the ray meets a node's grid on one axis: plane f = 1 + q / 32768
+// lies at t = step * f + near (or far), the offsets moved apart by the
+// rounding of (base - o) * inv (twice 2^-24 of it) and of the triangle
+// test's own translation by the origin, with room to spare: 2^-21 of a value
+// that is at least 32,768 quanta or the distance to the node.
+struct AxisPlanes {
+  float step, off_near, off_far;
+  uint32_t near_word, far_word;
+  PT_DEV AxisPlanes(float base, float grid, uint32_t lo, uint32_t hi, float o, float inv) {
+    const float slack = 4.76837158e-7f;
+    const float a = (base - o) * inv;
+    step = grid * inv;
+    off_near = fmaf(fabsf(a), -slack, a);
+    off_far = fmaf(fabsf(a), slack, a);
+    near_word = inv < 0.0f ? hi : lo;
+    far_word = inv < 0.0f ? lo : hi;
   }
+};
+
+// Both planes of child i on one axis by one packed multiply-add (each half
+// rounds as fmaf does).
+PT_DEV void near_far(const AxisPlanes &a, int i, float &n, float &f) {
+  unsigned long long p, st, off, r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(plane_at(a.near_word, i)), "f"(plane_at(a.far_word, i)));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(st) : "f"(a.step));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(off) : "f"(a.off_near), "f"(a.off_far));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(p), "l"(st), "l"(off));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(n), "=f"(f) : "l"(r));
+}
+// The hit children's sort keys: the entry distance's bits with the child
+// index in the low two (which child of two almost equally near ones comes
+// first decides nothing), all ones for a child the ray misses. A box counts
+// as hit when the ray enters it before it leaves it or t_far, either of them
+// widened by 2^-20 for the relative rounding of the plane distances and of a
+// candidate's own t. Rays start at t = 0. An unused slot is an empty leaf
+// with inverted planes: it needs no test of its own and does no harm where
+// its planes round together.
+PT_DEV uint32_t child_key(const AxisPlanes &x, const AxisPlanes &y, const AxisPlanes &z, int i, float t_far) {
+  float nx, ny, nz, fx, fy, fz;
+  near_far(x, i, nx, fx);
+  near_far(y, i, ny, fy);
+  near_far(z, i, nz, fz);
+  const float tn = max3f(nx, ny, fmaxf(nz, 0.0f));
+  const float tf = min3f(fx, fy, fminf(fz, t_far)) * 1.00000095f;
+  return tn <= tf ? (__float_as_uint(tn) & ~3u) | (uint32_t)i : 0xffffffffu;
 }
 
-// Tests the children of node `cur` and returns the nearest hit child
-// (kTravDone when none), pushing the other hit children farthest first.
-// Children are ordered by entry distance when `ordered`.
-PT_DEV int visit_node2(const DevScene &s, const Ray &r, float t_min, float t_far, int cur, int &sp, TravStack &stk,
-                       uint32_t &err, bool ordered) {
-  bool h0, h1;
-  float e0, e1;
-  int4 dd;
-  node_boxes(s.nodes + cur, r, t_min, t_far, h0, h1, e0, e1, dd);
-  if (h0 && h1) {
-    bool swap = ordered && e1 < e0;
-    stk.push(sp, swap ? dd.x : dd.y, err);
-    return swap ? dd.y : dd.x;
-  }
-  if (h0) return dd.x;
-  if (h1) return dd.y;
-  return kTravDone;
-}
-
-PT_DEV int visit_node4(const DevScene &s, const Ray &r, float t_min, float t_far, int cur, int &sp, TravStack &stk,
-                       uint32_t &err, bool ordered) {
-  const Bvh4Node *nd = s.nodes4 + cur;
-  const float4 lx = ldg4(&nd->lo_x), hx = ldg4(&nd->hi_x), ly = ldg4(&nd->lo_y), hy = ldg4(&nd->hi_y);
-  const float4 lz = ldg4(&nd->lo_z), hz = ldg4(&nd->hi_z);
-  const int4 ch = __ldg(&nd->child);
-  float e0, e1, e2, e3;
-  int c0 = child_box(lx.x, hx.x, ly.x, hy.x, lz.x, hz.x, r, t_min, t_far, e0) && ch.x != kEmptyChild ? ch.x : kTravDone;
-  int c1 = child_box(lx.y, hx.y, ly.y, hy.y, lz.y, hz.y, r, t_min, t_far, e1) && ch.y != kEmptyChild ? ch.y : kTravDone;
-  int c2 = child_box(lx.z, hx.z, ly.z, hy.z, lz.z, hz.z, r, t_min, t_far, e2) && ch.z != kEmptyChild ? ch.z : kTravDone;
-  int c3 = child_box(lx.w, hx.w, ly.w, hy.w, lz.w, hz.w, r, t_min, t_far, e3) && ch.w != kEmptyChild ? ch.w : kTravDone;
-  if (ordered) {
-    if (c0 == kTravDone) e0 = inf();
-    if (c1 == kTravDone) e1 = inf();
-    if (c2 == kTravDone) e2 = inf();
-    if (c3 == kTravDone) e3 = inf();
-    cswap(e0, c0, e1, c1);
-    cswap(e2, c2, e3, c3);
-    cswap(e0, c0, e2, c2);
-    cswap(e1, c1, e3, c3);
-    cswap(e1, c1, e2, c2);
-  }
-  int next = kTravDone;
-  if (c3 != kTravDone) next = c3;
-  if (c2 != kTravDone) {
-    if (next != kTravDone) stk.push(sp, next, err);
-    next = c2;
-  }
-  if (c1 != kTravDone) {
-    if (next != kTravDone) stk.push(sp, next, err);
-    next = c1;
-  }
-  if (c0 != kTravDone) {
-    if (next != kTravDone) stk.push(sp, next, err);
-    next = c0;
-  }
-  return next;
-}
-
-// Traversal position of one ray for speculative while-while traversal
-// (Aila & Laine 2009): in a warp's node phase every lane walks nodes; a lane
-// that reaches a leaf parks it in `leaf` and keeps walking until it meets a
-// second leaf, and the phase lasts while any lane is still looking for its
-// first one. The warp then tests the parked leaves together.
+// Traversal state of one ray. `cur` is the next node (>= 0), a leaf that
+// waits for the parked one (< 0) or kTravDone; `leaf` the parked leaf's
+// records still to test (first | count << kLeafCountShift). A leaf waits in
+// `cur` only while `leaf` holds records, but for the empty leaves of unused
+// child slots (settle).
+constexpr uint32_t kOneRecord = 1u << kLeafCountShift;
+template <int kThreads, bool kOnly4>
 struct TravCore {
-  Ray r;
-  int cur, sp, leaf;
+  V3 o, inv;
+  float sx, sy, sz;
+  uint32_t axes;  // kx | ky << 2 | kz << 4
+  const Bvh4Node *nodes4;
+  const BvhNode *nodes2;
+  const float4 *tris;
+  int cur;
+  uint32_t leaf;
+  float t_far;
   bool wide;
-  PT_DEV void start(const DevScene &s, V3 o, V3 d, bool wide_nodes) {
-    r = make_ray(o, d);
+
+  PT_DEV void start(const DevScene &s, V3 org, V3 dir, float tmax, bool wide_nodes, TravStack<kThreads> &stk,
+                    uint32_t words) {
+    const Ray r = make_ray(org, dir);
+    o = r.o;
+    inv = r.inv;
+    sx = r.sx;
+    sy = r.sy;
+    sz = r.sz;
+    axes = (uint32_t)(r.kx | r.ky << 2 | r.kz << 4);
+    nodes4 = s.nodes4;
+    nodes2 = s.nodes;
+    tris = s.tris;
     cur = s.node_count ? 0 : kTravDone;
-    sp = 0;
-    leaf = kTravDone;
+    leaf = 0;
+    t_far = tmax;
     wide = wide_nodes && s.nodes4;
+    stk.reset(words);
   }
-  PT_DEV bool searching() const { return leaf == kTravDone && (cur != kTravDone || sp > 0); }
-  // kTravDone is positive: "a node to visit" is cur >= 0 && cur != kTravDone.
-  PT_DEV bool can_step() const {
-    return leaf == kTravDone ? (cur != kTravDone || sp > 0)
-                             : ((cur >= 0 && cur != kTravDone) || (cur == kTravDone && sp > 0));
+  PT_DEV void idle() {
+    cur = kTravDone;
+    leaf = 0;
   }
-  PT_DEV bool finished() const { return leaf == kTravDone && cur == kTravDone && sp == 0; }
-  // One node-phase step; the caller checks can_step(). kOnly4: the caller
-  // knows the ray walks the four-child layout (`wide`), so the two-child
-  // visit is not compiled in.
-  template <bool kOnly4>
-  PT_DEV void node_step(const DevScene &s, float t_min, float t_far, TravStack &stk, uint32_t &nodes,
-                        uint32_t &err, bool ordered) {
-    if (cur < 0) {  // a leaf met in the previous node phase
-      leaf = cur;
-      cur = kTravDone;
-      return;
+  PT_DEV bool wants_node() const { return cur >= 0; }
+  PT_DEV bool wants_tri() const { return leaf >= kOneRecord; }
+  // A leaf in `cur` (not a node, not kTravDone).
+  PT_DEV bool leaf_waits() const { return (uint32_t)cur > 0x80000000u; }
+  // Parks the leaf in `cur` when no other is parked.
+  PT_DEV void settle(TravStack<kThreads> &stk, uint32_t words) {
+    if (leaf < kOneRecord && leaf_waits()) {
+      leaf = (uint32_t)~cur;
+      cur = stk.pop(words);
     }
-    if (cur == kTravDone) {
-      cur = stk.pop(sp);
-      if (cur == kTravDone) return;
-      if (cur < 0) {
-        if (leaf == kTravDone) {
-          leaf = cur;
-          cur = kTravDone;
+  }
+
+  // Visits node `cur`: the nearest hit child is next, the others go on the
+  // stack farthest first.
+  PT_DEV void node_step(TravStack<kThreads> &stk, uint32_t words, DevCounters *ctr) {
+    stk.count(words, ROW_NODES);
+    if (kOnly4 || wide) {
+      const Bvh4Node *nd = nodes4 + cur;
+      const float4 base = ldg4(&nd->base);
+      const uint4 mid = __ldg(&nd->mid), pl = __ldg(&nd->planes);
+      const int4 ch = __ldg(&nd->child);
+      const AxisPlanes x(base.x, base.w, mid.z, mid.w, o.x, inv.x);
+      const AxisPlanes y(base.y, __uint_as_float(mid.x), pl.x, pl.y, o.y, inv.y);
+      const AxisPlanes z(base.z, __uint_as_float(mid.y), pl.z, pl.w, o.z, inv.z);
+      const uint32_t none = 0xffffffffu;
+      const uint32_t k0 = child_key(x, y, z, 0, t_far), k1 = child_key(x, y, z, 1, t_far);
+      const uint32_t k2 = child_key(x, y, z, 2, t_far), k3 = child_key(x, y, z, 3, t_far);
+      const uint32_t a = min(k0, k1), b = max(k0, k1), c = min(k2, k3), d = max(k2, k3);
+      const uint32_t first = min(a, c), m0 = max(a, c), m1 = min(b, d), last = max(b, d);
+      const uint32_t second = min(m0, m1), third = max(m0, m1);
+      if (stk.room_for_three(words)) {
+        // Everything below stays in shared memory: no branches but the last.
+        if (third != none) {
+          stk.push_shared(last != none, child_of(ch, last));
+          stk.push_shared(true, child_of(ch, third));
+        }
+        stk.push_shared(second != none, child_of(ch, second));
+        cur = child_of(ch, first);
+        if (first == none) cur = stk.pop_shared();
+        if (leaf < kOneRecord && leaf_waits()) {
+          leaf = (uint32_t)~cur;
+          cur = stk.pop_shared();
         }
         return;
       }
+      if (last != none) stk.push(words, child_of(ch, last), ctr);
+      if (third != none) stk.push(words, child_of(ch, third), ctr);
+      if (second != none) stk.push(words, child_of(ch, second), ctr);
+      cur = first != none ? child_of(ch, first) : stk.pop(words);
+    } else {
+      Ray r;
+      r.o = o;
+      r.inv = inv;
+      bool h0, h1;
+      float e0, e1;
+      int4 dd;
+      node_boxes(nodes2 + cur, r, 0.0f, t_far, h0, h1, e0, e1, dd);
+      const bool swap = e1 < e0;
+      if (h0 && h1) stk.push(words, swap ? dd.x : dd.y, ctr);
+      cur = h0 && h1 ? (swap ? dd.y : dd.x) : (h0 ? dd.x : (h1 ? dd.y : stk.pop(words)));
     }
-    nodes++;
-    cur = kOnly4 || wide ? visit_node4(s, r, t_min, t_far, cur, sp, stk, err, ordered)
-                         : visit_node2(s, r, t_min, t_far, cur, sp, stk, err, ordered);
-    if (cur < 0 && leaf == kTravDone) {
-      leaf = cur;
-      cur = kTravDone;
-    }
+    settle(stk, words);
   }
-  // The parked leaf's triangle records [first, first + count).
-  PT_DEV void leaf_range(uint32_t &first, uint32_t &count) const {
-    first = (uint32_t)(~leaf);
-    count = first >> kLeafCountShift;
-    first &= kLeafFirstMask;
+
+  // Tests the parked leaf's next triangle. `hit(g, flags, t, b0, b1, b2,
+  // front)` is called for one that the ray meets at t >= 0.
+  template <class OnHit>
+  PT_DEV void tri_step(TravStack<kThreads> &stk, uint32_t words, const OnHit &hit) {
+    stk.count(words, ROW_TRIS);
+    const float4 *tr = tris + 3u * (leaf & kLeafFirstMask);
+    const float4 p0 = ldg4(tr), p1 = ldg4(tr + 1), p2 = ldg4(tr + 2);
+    leaf += 1u - kOneRecord;
+    Ray r;
+    r.o = o;
+    r.sx = sx;
+    r.sy = sy;
+    r.sz = sz;
+    r.kx = (int)(axes & 3u);
+    r.ky = (int)(axes >> 2 & 3u);
+    r.kz = (int)(axes >> 4);
+    float t, b0, b1, b2;
+    bool front;
+    if (intersect_watertight(r, {p0.x, p0.y, p0.z}, {p1.x, p1.y, p1.z}, {p2.x, p2.y, p2.z}, t, b0, b1, b2, front) &&
+        t >= 0.0f)
+      hit(__float_as_uint(p0.w), __float_as_uint(p1.w), t, b0, b1, b2, front);
+    settle(stk, words);
   }
 };
 
-// Closest-hit state of one ray.
-struct ClosestRay {
-  TravCore core;
-  float t_min, t_max;
-  Hit best;
-  bool have;
-  PT_DEV void init(const DevScene &s, V3 o, V3 d, float tmin, float tmax, bool wide_nodes) {
-    core.start(s, o, d, wide_nodes);
-    t_min = tmin;
-    t_max = tmax;
-    best.t = tmax;
-    best.g = 0xffffffffu;
-    have = false;
-  }
-  template <bool kOnly4>
-  PT_DEV void node_step(const DevScene &s, TravStack &stk, uint32_t &nodes, uint32_t &err) {
-    core.node_step<kOnly4>(s, t_min, best.t, stk, nodes, err, true);
-  }
-  // Tests the parked leaf (if any) and clears it.
-  template <class Accept>
-  PT_DEV void leaf_step(const DevScene &s, Accept &accept, uint32_t &tris) {
-    if (core.leaf == kTravDone) return;
-    uint32_t first, count;
-    core.leaf_range(first, count);
-    core.leaf = kTravDone;
-    for (uint32_t i = 0; i < count; ++i) {
-      const float4 *tr = s.tris + 3u * (first + i);
-      float4 p0 = ldg4(tr), p1 = ldg4(tr + 1), p2 = ldg4(tr + 2);
-      tris++;
-      float t, b0, b1, b2;
-      bool front;
-      if (!intersect_watertight(core.r, {p0.x, p0.y, p0.z}, {p1.x, p1.y, p1.z}, {p2.x, p2.y, p2.z}, t, b0, b1, b2,
-                                front))
-        continue;
-      if (!(t >= t_min)) continue;
-      uint32_t g = __float_as_uint(p0.w);
-      bool better = have ? (t < best.t || (t == best.t && g < best.g)) : (t <= t_max);
-      if (!better) continue;
-      if (accept(g, __float_as_uint(p1.w), t, b0, b1, b2, front)) {
-        best.t = t;
-        best.g = g;
-        best.b0 = b0;
-        best.b1 = b1;
-        best.b2 = b2;
-        best.front = front;
-        have = true;
-      }
-    }
-  }
+// A warp's share of the ray queue: entries [next, end) are claimed and not
+// yet handed out. Lives in shared memory, read and written by whole warps.
+struct WarpRun {
+  uint32_t next, end, exhausted;
 };
-
-// Any-hit state of one ray.
-struct ShadowTrav {
-  TravCore core;
-  float t_max;
-  bool occluded;
-  PT_DEV void init(const DevScene &s, V3 o, V3 d, float tmax, bool wide_nodes) {
-    core.start(s, o, d, wide_nodes);
-    t_max = tmax;
-    occluded = false;
-  }
-  template <bool kOnly4>
-  PT_DEV void node_step(const DevScene &s, TravStack &stk, uint32_t &nodes, uint32_t &err) {
-    core.node_step<kOnly4>(s, 0.0f, t_max, stk, nodes, err, false);
-  }
-  template <class Accept>
-  PT_DEV void leaf_step(const DevScene &s, Accept &accept, uint32_t &tris) {
-    if (core.leaf == kTravDone) return;
-    uint32_t first, count;
-    core.leaf_range(first, count);
-    core.leaf = kTravDone;
-    for (uint32_t i = 0; i < count; ++i) {
-      const float4 *tr = s.tris + 3u * (first + i);
-      float4 p0 = ldg4(tr), p1 = ldg4(tr + 1), p2 = ldg4(tr + 2);
-      tris++;
-      float t, b0, b1, b2;
-      bool front;
-      if (!intersect_watertight(core.r, {p0.x, p0.y, p0.z}, {p1.x, p1.y, p1.z}, {p2.x, p2.y, p2.z}, t, b0, b1, b2,
-                                front))
-        continue;
-      if (!(t >= 0.0f && t <= t_max)) continue;
-      if (accept(__float_as_uint(p0.w), __float_as_uint(p1.w), t, b0, b1, b2, front)) {
-        occluded = true;
-        return;
-      }
-    }
-  }
-  PT_DEV bool done() const { return occluded || core.finished(); }
-};
-
-// The node phase of while-while traversal ends once at most this many lanes
-// of the warp are still looking for their first leaf, instead of when the
-// last one finds it: the stragglers keep their traversal state and go on in
-// the next round, and the warp's other lanes test their parked leaves
-// meanwhile. Measured on the request mix: closest-hit traversal 701 -> 652
-// ms and shadow rays 519 -> 493 ms per step with 4 (2: 677 / 498, 8: 648 /
-// 487, 12: 672 / 496); on the sphere grid frame 36.6 -> 35.6 ms extend.
-// With the four-child-only kernels, 6 traced the mix 1 % faster than 4 and
-// the sphere grid frame within 0.2 %.
-constexpr int kNodePhaseStragglers = 6;
-
-// Warp-collective: whether the node phase goes on, given this lane's
-// `searching` (it has a ray and no parked leaf yet) and `ready` (it has a
-// parked leaf to test or a finished ray to write). The phase also goes on
-// while no lane is ready, so every round makes progress.
-PT_DEV bool node_phase_goes_on(bool searching, bool ready) {
-  const int n = __popc(__ballot_sync(0xffffffffu, searching));
-  return n > kNodePhaseStragglers || (n > 0 && !__any_sync(0xffffffffu, ready));
-}
-
-// Warp-aggregated claim of `chunk` consecutive queue entries for each lane
-// with `need`; returns this lane's first entry index (meaningful when
-// `need`). `exhausted` turns true (warp-uniformly) once the claims pass `n`,
-// after which no atomics are issued.
-PT_DEV uint32_t warp_claim(uint32_t *counter, bool need, uint32_t n, bool &exhausted, uint32_t chunk = 1) {
+// Hands each lane with `need` its next entry of the queue's `n` (warp
+// collective); true where one was taken. Claims `chunk` entries per lane
+// still without one.
+PT_DEV bool take_entry(WarpRun *run, uint32_t *counter, bool need, uint32_t n, uint32_t chunk, uint32_t &idx) {
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t mask = __ballot_sync(0xffffffffu, need);
-  if (mask == 0 || exhausted) return 0xffffffffu;
-  uint32_t leader = __ffs(mask) - 1;
-  uint32_t base = 0;
-  if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(mask) * chunk);
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (base + (uint32_t)__popc(mask) * chunk >= n) exhausted = true;
-  return base + (uint32_t)__popc(mask & ((1u << lane) - 1u)) * chunk;
-}
-
-// A lane's claimed queue entries not yet started: entries [next, next + left).
-struct ClaimedRun {
-  uint32_t next = 0, left = 0;
-  // Refills the run (warp-collective: every lane calls it) for lanes with
-  // no ray and no entries left, then hands out this lane's next entry in
-  // `idx` when it has no ray. Returns whether a new entry was taken.
-  PT_DEV bool take(uint32_t *counter, bool has, uint32_t n, bool &exhausted, uint32_t chunk, uint32_t &idx) {
-    const bool need = !has && left == 0;
-    const uint32_t first = warp_claim(counter, need, n, exhausted, chunk);
-    if (need && first < n) {
-      next = first;
-      left = min(chunk, n - first);
+  const uint32_t mask = __ballot_sync(0xffffffffu, need);
+  const uint32_t rank = __popc(mask & ((1u << lane) - 1u)), want = __popc(mask);
+  const uint32_t next = run->next, have = run->end - next;
+  uint32_t base = n, got = 0;
+  if (want > have && !run->exhausted) {
+    got = (want - have) * chunk;
+    if (lane == 0) base = atomicAdd(counter, got);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    got = base < n ? min(got, n - base) : 0u;
+  }
+  const uint32_t taken = min(want - min(want, have), got);  // of the new entries
+  __syncwarp();
+  if (lane == 0) {
+    if (want > have) {
+      run->next = base + taken;
+      run->end = base + got;
+      if (got < (want - have) * chunk) run->exhausted = 1u;
+    } else {
+      run->next = next + want;
     }
-    if (has || left == 0) return false;
-    idx = next++;
-    --left;
+  }
+  __syncwarp();
+  if (!need) return false;
+  if (rank < have) {
+    idx = next + rank;
     return true;
   }
-};
+  idx = base + (rank - have);
+  return rank - have < taken;
+}
 
 }  // namespace ptd

@@ -2,7 +2,7 @@
 //
 // HBM layout of one resident scene (all arrays 256-byte aligned):
 //   nodes     BvhNode[node_count]        64 B  two child boxes + child refs
-//   nodes4    Bvh4Node[node4_count]     128 B  the same tree, four children per node
+//   nodes4    Bvh4Node[node4_count]      64 B  the same tree, four children per node
 //   tris      float4[3 * tri_count]      48 B  leaf-ordered triangle records:
 //                                              (v0.xyz, global id), v1, v2
 //   tri_info  uint2[tri_count]            8 B  (material, attribute flags) by global id
@@ -32,17 +32,26 @@ struct alignas(16) BvhNode {
   int4 d;
 };
 
-// Four-child node, 128 bytes (one cache line), the same tree collapsed so
-// each node holds up to four children, boxes stored by axis:
-//   lo_x / hi_x / lo_y / hi_y / lo_z / hi_z  = that bound of children 0..3
-//   child = child refs as in BvhNode (>= 0 node, < 0 leaf), kEmptyChild
-//           for unused slots.
-struct alignas(128) Bvh4Node {
-  float4 lo_x, hi_x, lo_y, hi_y, lo_z, hi_z;
+// Four-child node, 64 bytes, the same tree collapsed so each node holds up
+// to four children, their boxes quantised to 8 bits a plane on a grid of the
+// node's own (pack_bvh4 in bvh4.h writes it):
+//   base    base.x, base.y, base.z, step.x
+//   mid     step.y, step.z (float bits), lower x planes, upper x planes
+//   planes  lower y, upper y, lower z, upper z
+//   child   child refs as in BvhNode (>= 0 node, < 0 leaf), kEmptyChild (a
+//           leaf of no triangles) for unused slots
+// Byte i of a plane word is child i's plane q, which lies at
+// base + step * (1 + q / 32768): step is a power of two, 32,768 quanta, so
+// 1 + q / 32768 is one byte placed inside the bits of 1.0f.
+// Half the bytes of full-precision boxes: a visit's scattered 16-byte loads
+// (the L1's scarce resource here) fall from seven to four, and twice the
+// nodes fit L1. Measured on closest-hit traversal: see k_wf_extend.
+struct alignas(64) Bvh4Node {
+  float4 base;
+  uint4 mid, planes;
   int4 child;
-  int4 pad;
 };
-constexpr int kEmptyChild = 0x7fffffff;
+constexpr int kEmptyChild = -1;
 // Node layout per ray kind in the wavefront (DevRequest::wide_nodes).
 enum WideNodes : uint32_t { WIDE_EXTENSION = 1u, WIDE_SHADOW = 2u };
 
@@ -135,6 +144,9 @@ struct WaveSegment {
   uint32_t sample_begin, spp;
   uint32_t pad0, pad1;
 };
+
+// WaveBuffers::hit_g: a path's hit of the current vertex.
+enum HitBits : uint32_t { HIT_FRONT = 1u << 31, HIT_FOUND = 1u << 30, HIT_G_MASK = (1u << 30) - 1u };
 
 // Structure-of-arrays path state of one wave of the wavefront schedule
 // (wavefront.cuh), `capacity` slots, `shadow_slots` queued shadow rays per

@@ -12,6 +12,7 @@
 // SAH-based Bounding Volume Hierarchies", 2007), built in parallel over
 // subtrees, emitted depth-first as two-child nodes.
 #include "host_scene.h"
+#include "bvh4.h"
 #include "bvh_build.h"
 #include "mip_build.h"
 
@@ -1026,25 +1027,29 @@ void emit_tree(const std::vector<BNode> &in_nodes, const std::vector<uint32_t> &
   // Four-child layout: a node starts from its two binary children and opens
   // the interior child of largest surface area until it holds four.
   {
-    auto set_child = [&](Bvh4Node &n, int slot, const BNode *c, int ref) {
-      float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-      if (c) pad_box(c->lo, c->hi, lo, hi);
-      reinterpret_cast<float *>(&n.lo_x)[slot] = lo[0];
-      reinterpret_cast<float *>(&n.hi_x)[slot] = hi[0];
-      reinterpret_cast<float *>(&n.lo_y)[slot] = lo[1];
-      reinterpret_cast<float *>(&n.hi_y)[slot] = hi[1];
-      reinterpret_cast<float *>(&n.lo_z)[slot] = lo[2];
-      reinterpret_cast<float *>(&n.hi_z)[slot] = hi[2];
-      reinterpret_cast<int *>(&n.child)[slot] = ref;
+    // The node over `children` (fewer than four: the rest stay unused).
+    auto pack = [&](const BNode *const children[4], const int ref[4]) {
+      float lo[3][4], hi[3][4];
+      for (int i = 0; i < 4; ++i) {
+        float l[3] = {INFINITY, INFINITY, INFINITY}, h[3] = {-INFINITY, -INFINITY, -INFINITY};
+        if (children[i]) pad_box(children[i]->lo, children[i]->hi, l, h);
+        for (int a = 0; a < 3; ++a) {
+          lo[a][i] = l[a];
+          hi[a][i] = h[a];
+        }
+      }
+      Bvh4Node n;
+      pack_bvh4(lo, hi, ref, n);
+      return n;
     };
     struct Item {
       uint32_t bin, gpu;
     };
     out_nodes4.push_back(Bvh4Node{});
-    out_nodes4[0].pad = make_int4(0, 0, 0, 0);
     if (root.count > 0) {
-      set_child(out_nodes4[0], 0, &root, leaf_ref(root.first, root.count));
-      for (int k = 1; k < 4; ++k) set_child(out_nodes4[0], k, nullptr, kEmptyChild);
+      const BNode *const only[4] = {&root, nullptr, nullptr, nullptr};
+      const int ref[4] = {leaf_ref(root.first, root.count), kEmptyChild, kEmptyChild, kEmptyChild};
+      out_nodes4[0] = pack(only, ref);
     } else {
       std::vector<Item> st{{0, 0}};
       while (!st.empty()) {
@@ -1073,23 +1078,20 @@ void emit_tree(const std::vector<BNode> &in_nodes, const std::vector<uint32_t> &
           ++nch;
         }
         std::vector<Item> next;
-        for (int k = 0; k < 4; ++k) {
-          if (k >= nch) {
-            set_child(out_nodes4[it.gpu], k, nullptr, kEmptyChild);
-            continue;
-          }
+        const BNode *cs[4] = {};
+        int ref[4] = {kEmptyChild, kEmptyChild, kEmptyChild, kEmptyChild};
+        for (int k = 0; k < nch; ++k) {
           const BNode &c = nodes[ch[k]];
-          int ref;
+          cs[k] = &c;
           if (c.count > 0) {
-            ref = leaf_ref(c.first, c.count);
+            ref[k] = leaf_ref(c.first, c.count);
           } else {
-            ref = (int)out_nodes4.size();
+            ref[k] = (int)out_nodes4.size();
             out_nodes4.push_back(Bvh4Node{});
-            out_nodes4.back().pad = make_int4(0, 0, 0, 0);
-            next.push_back({ch[k], (uint32_t)ref});
+            next.push_back({ch[k], (uint32_t)ref[k]});
           }
-          set_child(out_nodes4[it.gpu], k, &c, ref);
         }
+        out_nodes4[it.gpu] = pack(cs, ref);
         for (auto r = next.rbegin(); r != next.rend(); ++r) st.push_back(*r);
       }
     }

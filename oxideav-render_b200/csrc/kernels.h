@@ -32,6 +32,17 @@ cudaError_t launch_megakernel(const DevRequest *reqs, const WaveSegment *segs, u
 // written on `st` beforehand.
 cudaError_t launch_wavefront(const WaveBuffers &w, DevCounters *ctr, int num_sms, cudaStream_t st,
                              StageTimer *timer = nullptr, bool accumulate = true);
+// One iteration's traversal launches (trace.cu). prepare_trace_kernels
+// queries their occupancy, which must not happen inside a stream capture.
+void prepare_trace_kernels();
+void launch_wf_extend(const WaveBuffers &w, uint32_t it, DevCounters *ctr, int num_sms, cudaStream_t st);
+// One iteration's shading launch at three or four blocks per SM (shade3.cu,
+// shade4.cu), and the constant table each of them keeps.
+void launch_wf_shade3(const WaveBuffers &w, uint32_t it, uint32_t grid, cudaStream_t st);
+void launch_wf_shade4(const WaveBuffers &w, uint32_t it, uint32_t grid, cudaStream_t st);
+cudaError_t set_shade3_tables(const float *sheen_lut);
+cudaError_t set_shade4_tables(const float *sheen_lut);
+void launch_wf_shadow(const WaveBuffers &w, uint32_t it, DevCounters *ctr, int num_sms, cudaStream_t st);
 // The in-order accumulate of a traced wave on its own (k_wf_accumulate).
 cudaError_t launch_wave_accumulate(const WaveBuffers &w, int num_sms, cudaStream_t st);
 // The same launch sequence captured once as an executable CUDA graph; it

@@ -83,6 +83,7 @@ SIGNATURES = {
     # include/pt_b200_debug.h
     "pt_set_bvh_builder": (i32, [vp, u32]),
     "pt_debug_build_bvh": (i32, [fp, u32, u32, dp, vp, u64, vp, u64]),
+    "pt_debug_pack_node4": (i32, [fp, fp, C.POINTER(C.c_int32), u32p]),
     "pt_scene_bvh_on_device": (i32, [vp, u32, C.POINTER(C.c_int)]),
     "pt_scene_upload_seconds": (i32, [vp, u32, dp]),
     "pt_debug_scene_texels": (i32, [vp, u32, fp, u64, u64p]),
