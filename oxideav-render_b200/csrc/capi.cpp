@@ -145,6 +145,7 @@ Job make_job(const pt_tracer &t, const SceneHost &sc, const EnvHost *env, uint32
   j.iterations = t.opts.path_trace.max_bounces + 1;
   j.shadow_slots = sc.light_count + 1;
   j.scene_key = t.scene_id;
+  j.layered = sc.dev.layered != 0;
   j.area = sc.dev.em_count > 0 || env != nullptr;
   j.wide = sc.dev.nodes4 ? j.req.wide_nodes & (uint32_t)(WIDE_EXTENSION | WIDE_SHADOW) : 0u;
   return j;
@@ -348,14 +349,15 @@ pt_status run_jobs(pt_context *ctx, std::vector<pt_tracer *> &tracers, std::vect
   if (overlap && (st = engine_overlap_begin(ctx)) != PT_OK) return st;
   for (size_t i = 0; i < waves.size(); ++i) {
     uint32_t iters = 1, wide = WIDE_EXTENSION | WIDE_SHADOW;
-    bool area = false;
+    bool area = false, layered = false;
     for (const WaveSegment &s : waves[i]) {
       iters = std::max(iters, jobs[s.request].iterations);
       area = area || jobs[s.request].area;
+      layered = layered || jobs[s.request].layered;
       wide &= jobs[s.request].wide;
     }
     st = launch_wave(ctx, ctx->d_reqs, ctx->d_segs + first_seg[i], waves[i], iters, &timer,
-                     overlap ? (int)(i % ctx->overlap_arenas) : -1, area, wide);
+                     overlap ? (int)(i % ctx->overlap_arenas) : -1, area, wide, layered);
     if (st != PT_OK) return st;
   }
   timer.mark(STAGE_END, ctx->stream);
@@ -728,7 +730,7 @@ pt_status engine_overlap_begin(pt_context *ctx) {
 
 pt_status launch_wave(pt_context *ctx, const DevRequest *d_reqs, const WaveSegment *d_segs,
                       const std::vector<WaveSegment> &segs, uint32_t iters, StageTimer *timer, int arena,
-                      bool area, uint32_t all_wide) {
+                      bool area, uint32_t all_wide, bool layered) {
   uint32_t nseg = (uint32_t)segs.size(), total = 0, max_pix = 0;
   for (const WaveSegment &s : segs) {
     total += s.pixel_count * s.spp;
@@ -743,6 +745,7 @@ pt_status launch_wave(pt_context *ctx, const DevRequest *d_reqs, const WaveSegme
     w.shade_blocks = ctx->shade_blocks == 4 ? 4u : 3u;
     w.trav_threads = ctx->trav_threads == 128 ? 128u : 256u;
     w.claim_chunk = ctx->claim_chunk == 2 || ctx->claim_chunk == 4 ? ctx->claim_chunk : 1u;
+    w.layered = layered ? 1u : 0u;
     w.all_wide = all_wide & (uint32_t)(WIDE_EXTENSION | WIDE_SHADOW);
     cudaStream_t ws = own_stream ? ctx->wave_streams[arena] : ctx->stream;
     // The arena's previous wave must be accumulated before this one
@@ -759,7 +762,7 @@ pt_status launch_wave(pt_context *ctx, const DevRequest *d_reqs, const WaveSegme
       // launch instead of ~6 per bounce.
       const uint32_t key = iters << 12 | w.all_wide << 10 | w.claim_chunk << 7 | (w.trav_threads == 128 ? 64u : 0u) |
                            (own_stream ? 4u * (1u + (uint32_t)arena) : 0u) | (w.shade_blocks == 4 ? 2u : 0u) |
-                           w.sort_materials;
+                           (w.layered ? 32u : 0u) | w.sort_materials;
       auto it = ctx->graphs.find(key);
       if (it == ctx->graphs.end()) {
         cudaGraphExec_t ge = nullptr;

@@ -318,7 +318,12 @@ struct NeeInput {
 // emission MIS pdf come from `pre` instead of being computed here, which
 // keeps the f64 spherical-triangle and environment sampling code out of
 // this (large) function's instruction footprint.
-template <class Sink, bool kPre = false>
+//
+// kPlain: the hit's material is TRI_PLAIN (or the ray missed). The layered
+// lobes' weights are then constants, which the compiler folds through the
+// same expressions: the same values from a fraction of the registers and
+// instructions.
+template <class Sink, bool kPre = false, bool kPlain = false>
 PT_DEV bool shade(const DevRequest &rq, PathState &ps, bool found, const Hit &hit, Sink &sink,
                   const NeeInput *pre = nullptr) {
   const DevScene &s = *rq.scene;
@@ -389,7 +394,7 @@ PT_DEV bool shade(const DevRequest &rq, PathState &ps, bool found, const Hit &hi
   }
   const bool flip = !hit.front && ds;
   MaterialSample mat;
-  material_oriented(s, dm, hit.g, flags, hit.b0, hit.b1, hit.b2, surf.sn, lod, flip, mat);
+  material_oriented<false, kPlain>(s, dm, hit.g, flags, hit.b0, hit.b1, hit.b2, surf.sn, lod, flip, mat);
   if (flip) {
     mat.normal = vneg(mat.normal);
     mat.clearcoat_normal = vneg(mat.clearcoat_normal);

@@ -303,19 +303,19 @@ PT_DEV Surface surface(const DevScene &s, uint32_t g, float b0, float b1, float 
 }
 
 // ---------------------------------------------------------------- textures
-PT_DEV uint32_t wrap_index(int64_t i, int64_t n, uint32_t mode) {
-  int64_t r;
-  if (mode == PT_WRAP_REPEAT) {
-    r = i % n;
-    if (r < 0) r += n;
-  } else if (mode == PT_WRAP_CLAMP) {
-    r = i < 0 ? 0 : (i > n - 1 ? n - 1 : i);
-  } else {
-    int64_t m = i % (2 * n);
-    if (m < 0) m += 2 * n;
-    r = m >= n ? 2 * n - 1 - m : m;
-  }
-  return (uint32_t)r;
+// Texel index i wrapped into n texels. filter_level clamps the coordinate to
+// 1e6 repeats, so i / period is known to within 0.3 from f32 and the
+// remainder follows in 32-bit arithmetic with one correction either way: a
+// 64-bit division is some hundred instructions, inlined at every lookup of
+// every texture binding.
+PT_DEV uint32_t wrap_index(int64_t i, uint32_t n, uint32_t mode) {
+  if (mode == PT_WRAP_CLAMP) return i < 0 ? 0u : (i > (int64_t)n - 1 ? n - 1u : (uint32_t)i);
+  const int32_t period = (int32_t)(mode == PT_WRAP_REPEAT ? n : 2u * n);
+  const int32_t q = (int32_t)floorf((float)i * __frcp_rn((float)period));
+  int32_t r = (int32_t)((uint32_t)i - (uint32_t)q * (uint32_t)period);
+  if (r < 0) r += period;
+  if (r >= period) r -= period;
+  return r >= (int32_t)n ? (uint32_t)(period - 1 - r) : (uint32_t)r;
 }
 PT_DEV float4 lerp4(float4 a, float4 b, float t) {
   return make_float4(a.x + (b.x - a.x) * t, a.y + (b.y - a.y) * t, a.z + (b.z - a.z) * t, a.w + (b.w - a.w) * t);
@@ -345,25 +345,33 @@ PT_DEV float4 filter_level(const float4 *texels, uint32_t w, uint32_t h, float u
 // PreparedTexture::sample_lod, src/texture.rs:420-451.
 PT_DEV float4 sample_lod(const DevScene &s, const DevTexture &t, float u, float v, float lod, bool srgb) {
   const uint64_t *off = srgb ? t.srgb_off : t.lin_off;
-  if (isnan(lod) || lod <= 0.0f)
-    return filter_level(s.texels + off[0], t.lw[0], t.lh[0], u, v, t.mag == PT_FILTER_LINEAR, t.wrap_s, t.wrap_t);
-  uint32_t mn = t.min;
-  bool lin = (mn == PT_MIN_LINEAR || mn == PT_MIN_LINEAR_MIP_NEAREST || mn == PT_MIN_LINEAR_MIP_LINEAR);
-  float max_level = (float)(t.levels - 1);
-  if (mn == PT_MIN_NEAREST || mn == PT_MIN_LINEAR)
-    return filter_level(s.texels + off[0], t.lw[0], t.lh[0], u, v, lin, t.wrap_s, t.wrap_t);
-  if (mn == PT_MIN_NEAREST_MIP_NEAREST || mn == PT_MIN_LINEAR_MIP_NEAREST) {
-    uint32_t l = f2u32(clampr(roundf(lod), 0.0f, max_level));
-    return filter_level(s.texels + off[l], t.lw[l], t.lh[l], u, v, lin, t.wrap_s, t.wrap_t);
+  const uint32_t mn = t.min;
+  const bool magnify = isnan(lod) || lod <= 0.0f;
+  const bool lin = magnify ? t.mag == PT_FILTER_LINEAR
+                           : (mn == PT_MIN_LINEAR || mn == PT_MIN_LINEAR_MIP_NEAREST || mn == PT_MIN_LINEAR_MIP_LINEAR);
+  // One level, or two and the blend between them, through one filter_level.
+  uint32_t l0 = 0, l1 = 0;
+  float f = 0.0f;
+  if (!magnify && mn != PT_MIN_NEAREST && mn != PT_MIN_LINEAR) {
+    const float max_level = (float)(t.levels - 1);
+    if (mn == PT_MIN_NEAREST_MIP_NEAREST || mn == PT_MIN_LINEAR_MIP_NEAREST) {
+      l0 = l1 = f2u32(clampr(roundf(lod), 0.0f, max_level));
+    } else {
+      const float l = clampr(lod, 0.0f, max_level);
+      l0 = f2u32(floorf(l));
+      l1 = min(l0 + 1, t.levels - 1);
+      f = l - (float)l0;
+    }
   }
-  float l = clampr(lod, 0.0f, max_level);
-  uint32_t l0 = f2u32(floorf(l));
-  uint32_t l1 = min(l0 + 1, t.levels - 1);
-  float f = l - (float)l0;
-  float4 a = filter_level(s.texels + off[l0], t.lw[l0], t.lh[l0], u, v, lin, t.wrap_s, t.wrap_t);
-  if (f <= 0.0f || l0 == l1) return a;
-  float4 b = filter_level(s.texels + off[l1], t.lw[l1], t.lh[l1], u, v, lin, t.wrap_s, t.wrap_t);
-  return lerp4(a, b, f);
+  const bool blend = f > 0.0f && l0 != l1;
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+  for (uint32_t l = l0;; l = l1) {
+    const float4 c = filter_level(s.texels + off[l], t.lw[l], t.lh[l], u, v, lin, t.wrap_s, t.wrap_t);
+    if (!blend) return c;
+    if (l == l1) return lerp4(a, c, f);
+    a = c;
+  }
 }
 
 // Texture LOD of a hit: ray cone at the camera vertex, level 0 after.
@@ -502,8 +510,9 @@ PT_DEV float fin(float v, float d) { return isfinite(v) ? v : d; }
 
 // TraceScene::material_oriented, src/trace.rs:700-923 (the occlusion
 // input is evaluated only when kOcclusion is set: the path tracer never
-// reads it).
-template <bool kOcclusion = false, class Lod>
+// reads it). kPlain: the material has no extension that adds a lobe or a
+// medium (TRI_PLAIN), so the inputs of those are their constants.
+template <bool kOcclusion = false, bool kPlain = false, class Lod>
 PT_DEV void material_oriented(const DevScene &s, const DevMaterial &dm, uint32_t g, uint32_t flags, float b0, float b1,
                               float b2, V3 shading_normal, const Lod &lod, bool flip, MaterialSample &m) {
   const pt_material &mat = dm.m;
@@ -543,7 +552,7 @@ PT_DEV void material_oriented(const DevScene &s, const DevMaterial &dm, uint32_t
     emissive.y *= t.y;
     emissive.z *= t.z;
   }
-  uint32_t ext = mat.ext_flags;
+  const uint32_t ext = kPlain ? mat.ext_flags & PT_EXT_SPECULAR : mat.ext_flags;
   float specular = 1.0f;
   V3 specular_color = {1.0f, 1.0f, 1.0f};
   if (ext & PT_EXT_SPECULAR) {

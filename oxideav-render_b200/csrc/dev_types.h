@@ -60,6 +60,9 @@ enum TriFlags : uint32_t {
   TRI_HAS_TANGENTS = 1u << 1,
   TRI_HAS_COLORS = 1u << 2,
   TRI_UV0 = 1u << 3,          // TRI_UV0 << s: UV set s present
+  // The material has metallic-roughness lobes only (of the extensions at most
+  // specular, ior, unlit and emissive strength).
+  TRI_PLAIN = 1u << 16,
 };
 
 // Triangle record flags (second record's w): what the any-hit filter needs
@@ -107,6 +110,7 @@ struct DevScene {
   const uint32_t *em_lookup;
   uint32_t node_count, tri_count, material_count, texture_count, light_count, em_count;
   uint32_t max_depth, node4_count;
+  uint32_t layered, pad;   // layered: some triangle is not TRI_PLAIN
   const Bvh4Node *nodes4;  // the same tree with four-child nodes
 };
 
@@ -153,7 +157,8 @@ enum HitBits : uint32_t { HIT_FRONT = 1u << 31, HIT_FOUND = 1u << 30, HIT_G_MASK
 // slot.
 // Per iteration: [0] active count, [1] shadow-queue count, [2] extend claim
 // cursor, [3] shadow claim cursor, [4] most shadow rays of a queued path,
-// [5..7] spare.
+// [5] sorted-queue entries before the first of a layered material,
+// [6..7] spare.
 constexpr uint32_t kWfCounterStride = 8;
 
 struct WaveBuffers {
@@ -176,6 +181,7 @@ struct WaveBuffers {
   uint32_t shade_blocks;       // 3 or 4: the k_wf_shade instantiation (blocks per SM)
   uint32_t trav_threads;       // 128 or 256: block size of the traversal kernels (1,024 threads per SM)
   uint32_t claim_chunk;        // 1, 2 or 4: queue entries a traversal lane claims per refill
+  uint32_t layered;            // some request of the wave has layered materials (host-side launch choice)
   uint32_t all_wide;           // WIDE_* bits that hold for every request of the wave (host-side launch choice)
 };
 
@@ -189,7 +195,9 @@ struct WaveDesc {
   uint32_t flags;  // WAVE_AREA_LIGHTS: some request has emissive triangles or an environment
 };
 enum WaveFlags : uint32_t { WAVE_AREA_LIGHTS = 1u };
-constexpr uint32_t kSortBuckets = 256;
+// Material-sort buckets: 0 misses, then those of plain materials, from
+// kLayeredBucket on those of layered ones.
+constexpr uint32_t kSortBuckets = 256, kLayeredBucket = 128;
 
 // Per-launch device counters (rays traced, traversal work, errors).
 struct DevCounters {

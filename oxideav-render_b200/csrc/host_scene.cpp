@@ -1490,6 +1490,7 @@ std::string build_scene_image(const pt_scene_desc &desc, SceneImage &img, bool w
   copy_task(plan.off[p_pmf], pmf.data(), plan.bytes[p_pmf]);
   copy_task(plan.off[p_cdf], cdf.data(), plan.bytes[p_cdf]);
   copy_task(plan.off[p_desc], nullptr, plan.bytes[p_desc]);
+  bool layered = false;
   // Corner streams by global triangle id: each item's array, or zeros for
   // an item without it.
   for (uint32_t i = 0; i < desc.item_count; ++i) {
@@ -1512,6 +1513,10 @@ std::string build_scene_image(const pt_scene_desc &desc, SceneImage &img, bool w
     for (int s = 0; s < PT_MAX_UV_SETS; ++s)
       if (it.uvs[s]) flags |= TRI_UV0 << s;
     const pt_material &mm = desc.materials[it.material];
+    if (!(mm.ext_flags & ~(uint32_t)PT_EXT_SPECULAR))
+      flags |= TRI_PLAIN;
+    else if (n > 0)
+      layered = true;
     const uint32_t rf = (mm.alpha_mode == PT_ALPHA_OPAQUE ? REC_OPAQUE : 0u) | (mm.double_sided ? REC_DOUBLE_SIDED : 0u);
     const uint2 inf = make_uint2(it.material, flags);
     uint2 *info = reinterpret_cast<uint2 *>(dst + plan.off[p_info]);
@@ -1571,6 +1576,7 @@ std::string build_scene_image(const pt_scene_desc &desc, SceneImage &img, bool w
   auto rel = [&](size_t part, size_t bytes) -> uintptr_t { return bytes ? (uintptr_t)plan.off[part] + 1 : 0; };
   DevScene &d = img.rel;
   std::memset(&d, 0, sizeof d);
+  d.layered = layered ? 1u : 0u;
   d.tri_info = (const uint2 *)rel(p_info, 1);
   d.pos = (const float *)rel(p_pos, 1);
   d.nrm = (const float *)rel(p_nrm, plan.bytes[p_nrm]);

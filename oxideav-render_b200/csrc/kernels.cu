@@ -295,6 +295,7 @@ __global__ void k_debug_bsdf(const float *params, const float *dirs, const float
 cudaError_t set_tables(const float *sheen_lut, const float *srgb_thresh) {
   cudaError_t e = cudaMemcpyToSymbol(g_sheen_lut, sheen_lut, sizeof(float) * SHEEN_LUT_COS * SHEEN_LUT_ROUGH);
   // The table is per translation unit that shades.
+  if (e == cudaSuccess) e = set_shade_plain_tables(sheen_lut);
   if (e == cudaSuccess) e = set_shade3_tables(sheen_lut);
   if (e == cudaSuccess) e = set_shade4_tables(sheen_lut);
   if (e != cudaSuccess) return e;
@@ -317,8 +318,7 @@ cudaError_t launch_wavefront(const WaveBuffers &w, DevCounters *ctr, int num_sms
   if (e == cudaSuccess && w.sort_materials)
     e = cudaMemsetAsync(w.sort_counts, 0, sizeof(uint32_t) * 2 * kSortBuckets * (w.iterations + 1), st);
   if (e != cudaSuccess) return e;
-  const bool shade4 = w.shade_blocks == 4;
-  const uint32_t g_shade = (uint32_t)num_sms * (shade4 ? 8 : 6), g_wide = (uint32_t)num_sms * 16,
+  const uint32_t g_sort = (uint32_t)num_sms * 6, g_wide = (uint32_t)num_sms * 16,
                  g_nee = (uint32_t)num_sms * 8;
   tm.mark(STAGE_RAYGEN, st);
   k_wf_raygen<<<g_wide, 256, 0, st>>>(w);
@@ -327,17 +327,20 @@ cudaError_t launch_wavefront(const WaveBuffers &w, DevCounters *ctr, int num_sms
     launch_wf_extend(w, it, ctr, num_sms, st);
     if (w.sort_materials) {
       tm.mark(STAGE_SORT, st);
-      k_wf_sort_count<<<g_shade, 256, 0, st>>>(w, it);
+      k_wf_sort_count<<<g_sort, 256, 0, st>>>(w, it);
       k_wf_sort_scan<<<1, kSortBuckets, 0, st>>>(w, it);
-      k_wf_sort_scatter<<<g_shade, 256, 0, st>>>(w, it);
+      k_wf_sort_scatter<<<g_sort, 256, 0, st>>>(w, it);
     }
     tm.mark(STAGE_NEE, st);
     k_wf_nee<<<g_nee, 256, 0, st>>>(w, it);
     tm.mark(STAGE_SHADE, st);
-    if (shade4)
-      launch_wf_shade4(w, it, g_shade, st);
-    else
-      launch_wf_shade3(w, it, g_shade, st);
+    if (w.sort_materials) launch_wf_shade_plain(w, it, num_sms, st);
+    if (w.layered || !w.sort_materials) {
+      if (w.shade_blocks == 4)
+        launch_wf_shade4(w, it, num_sms, st);
+      else
+        launch_wf_shade3(w, it, num_sms, st);
+    }
     tm.mark(STAGE_SHADOW, st);
     launch_wf_shadow(w, it, ctr, num_sms, st);
     k_wf_shadow_add<<<g_wide, 256, 0, st>>>(w, it);

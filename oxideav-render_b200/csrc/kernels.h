@@ -36,10 +36,13 @@ cudaError_t launch_wavefront(const WaveBuffers &w, DevCounters *ctr, int num_sms
 // queries their occupancy, which must not happen inside a stream capture.
 void prepare_trace_kernels();
 void launch_wf_extend(const WaveBuffers &w, uint32_t it, DevCounters *ctr, int num_sms, cudaStream_t st);
-// One iteration's shading launch at three or four blocks per SM (shade3.cu,
-// shade4.cu), and the constant table each of them keeps.
-void launch_wf_shade3(const WaveBuffers &w, uint32_t it, uint32_t grid, cudaStream_t st);
-void launch_wf_shade4(const WaveBuffers &w, uint32_t it, uint32_t grid, cudaStream_t st);
+// One iteration's shading launches: the plain materials (of a sorted queue),
+// and the layered ones at 384 or 512 threads per SM; and the constant table
+// that each translation unit keeps.
+void launch_wf_shade_plain(const WaveBuffers &w, uint32_t it, int num_sms, cudaStream_t st);
+void launch_wf_shade3(const WaveBuffers &w, uint32_t it, int num_sms, cudaStream_t st);
+void launch_wf_shade4(const WaveBuffers &w, uint32_t it, int num_sms, cudaStream_t st);
+cudaError_t set_shade_plain_tables(const float *sheen_lut);
 cudaError_t set_shade3_tables(const float *sheen_lut);
 cudaError_t set_shade4_tables(const float *sheen_lut);
 void launch_wf_shadow(const WaveBuffers &w, uint32_t it, DevCounters *ctr, int num_sms, cudaStream_t st);

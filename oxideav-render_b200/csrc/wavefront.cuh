@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(256) k_wf_raygen(WaveBuffers w) {
     uint32_t y = p / rq.width, x = p - y * rq.width;
     PathState ps;
     init_path(rq, x, y, seg.sample_begin + sidx, ps);
-    wf_store(w, slot, ps, seg.request);
+    wf_store_camera(w, slot, ps, seg.request);
     w.q[0][slot] = slot;
   }
 }
@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kSortBuckets) k_wf_sort_scan(WaveBuffers w, ui
     __syncthreads();
   }
   count[kSortBuckets + t] = s[t] - own;
+  if (t == kLayeredBucket) w.counters[iter * kWfCounterStride + 5] = s[t] - own;
 }
 
 __global__ void __launch_bounds__(256) k_wf_sort_scatter(WaveBuffers w, uint32_t iter) {
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_nee(WaveBuffers w, uint32_t iter)
     const DevRequest &rq = reqs[sd.w];
     const DevScene &s = *rq.scene;
     if (!rq.env && s.em_count == 0) continue;  // shade reads nothing for this request
-    const uint32_t k = __float_as_uint(w.o[slot].w);
+    const uint32_t k = iter;  // every queued path is at this vertex
     const uint32_t g = hg & HIT_G_MASK;
     const float4 tb = w.hit_tb[slot];
     const V3 pos = interp3(s.pos, g, tb.y, tb.z, tb.w);

@@ -64,9 +64,9 @@ PT_DEV bool accept_candidate(const WaveBuffers &w, uint32_t slot, uint32_t ray, 
 // The material-sort key of a ray that hit (a miss has key 0), stored by queue position, so the
 // count / scatter passes read keys and slots contiguously.
 PT_DEV uint32_t sort_key(const DevScene *s, uint32_t g) {
-  uint32_t m = __ldg(s->tri_info + g).x;
-  uint32_t sh = (uint32_t)((uintptr_t)s >> 8) * 0x9E3779B1u;
-  return 1u + (m + sh) % (kSortBuckets - 1u);
+  const uint2 info = __ldg(s->tri_info + g);
+  const uint32_t h = info.x + (uint32_t)((uintptr_t)s >> 8) * 0x9E3779B1u;
+  return (info.y & TRI_PLAIN) ? 1u + h % (kLayeredBucket - 1u) : kLayeredBucket + h % (kSortBuckets - kLayeredBucket);
 }
 
 // Closest hit of every queued path: persistent lanes, one ray each, refilled
