@@ -280,6 +280,25 @@ pt_status ensure_wavefront(pt_context *ctx, uint32_t capacity, uint32_t shadow_s
   return PT_OK;
 }
 
+// Paths of a refine up to which the megakernel runs it, where nobody chose
+// the schedule. A wavefront wave is some seventy short launches whatever its
+// size; up to about one resident set of threads (148 SMs x 384) a path's own
+// chain of vertices is shorter. Device and wall time of one refine, 8 bounces,
+// wavefront / megakernel in ms: without area lights (sphere grid, material
+// extensions) 16 K paths 1.06 / 0.53 and 1.20 / 0.52, 64 K 1.28 / 0.71 and
+// 1.36 / 0.78, 131 K 1.41 / 1.15 and 1.34 / 1.25, 262 K 1.62 / 1.96 and 1.44 /
+// 2.12; with them (Cornell box, 100k soup: the f64 sampling is in its loop)
+// 4 K 0.74 / 0.37 and 2.55 / 2.43, 16 K 0.80 / 0.48 and 2.83 / 2.64, 32 K
+// 0.84 / 0.83 and 3.13 / 2.97, 64 K 0.87 / 1.21 and 3.30 / 4.68.
+constexpr uint64_t kSmallRefine = 96u << 10, kSmallRefineArea = 24u << 10;
+
+// Restores the context's schedule after a small refine.
+struct ScheduleScope {
+  pt_context *ctx;
+  uint32_t schedule;
+  ~ScheduleScope() { ctx->schedule = schedule; }
+};
+
 // Runs a batch of refine jobs in merged waves: every wave carries path
 // slots of several tracers, each path reading its own request (scene,
 // camera, options, accumulator). Per-sample radiance is a pure function of
@@ -318,6 +337,12 @@ pt_status run_jobs(pt_context *ctx, std::vector<pt_tracer *> &tracers, std::vect
       flat.push_back(s);
     }
     max_slots = std::max(max_slots, slots);
+  }
+  ScheduleScope scope{ctx, ctx->schedule};
+  if (ctx->schedule == PT_SCHEDULE_WAVEFRONT && !ctx->schedule_fixed && !ctx->stage_timing && waves.size() == 1) {
+    bool area = false;
+    for (const Job &jb : jobs) area = area || jb.area;
+    if (max_slots <= (area ? kSmallRefineArea : kSmallRefine)) ctx->schedule = PT_SCHEDULE_MEGAKERNEL;
   }
   // Overlapped waves need the wavefront, two or more waves, and no per-stage
   // timing (whose events sit on one stream).
@@ -424,13 +449,14 @@ pt_status add_job(pt_context *ctx, pt_tracer *t, uint32_t n, std::vector<pt_trac
 struct KnobScope {
   pt_context *ctx;
   uint32_t schedule, wave_slots, shade_blocks, arenas, trav_threads, claim_chunk;
-  bool sort;
+  bool sort, fixed;
   KnobScope(pt_context *c, const TuneChoice *tc)
       : ctx(c), schedule(c->schedule), wave_slots(c->wave_slots), shade_blocks(c->shade_blocks),
         arenas(c->overlap_arenas), trav_threads(c->trav_threads), claim_chunk(c->claim_chunk),
-        sort(c->material_sort) {
+        sort(c->material_sort), fixed(c->schedule_fixed) {
     if (tc) {
       c->schedule = tc->schedule;
+      c->schedule_fixed = true;
       c->wave_slots = tc->wave_slots;
       c->material_sort = tc->material_sort != 0;
       c->shade_blocks = tc->shade_blocks;
@@ -443,6 +469,7 @@ struct KnobScope {
   }
   ~KnobScope() {
     ctx->schedule = schedule;
+    ctx->schedule_fixed = fixed;
     ctx->wave_slots = wave_slots;
     ctx->material_sort = sort;
     ctx->shade_blocks = shade_blocks;
@@ -505,6 +532,7 @@ pt_status autotune_scene(pt_context *ctx, const pt_tracer *t, SceneHost *sc, con
     for (uint32_t sort : {1u, 0u})
       for (uint32_t slots : {1u << 23, 1u << 20}) cands.push_back({PT_SCHEDULE_WAVEFRONT, wide, sort, slots, 0.0f});
   KnobScope restore(ctx, nullptr);
+  ctx->schedule_fixed = true;
   best = cands[0];
   float best_ms = -1.0f;
   auto time_choice = [&](TuneChoice &c, float &ms, uint32_t spp) -> pt_status {
@@ -1267,12 +1295,14 @@ pt_status pt_set_schedule(pt_context *ctx, uint32_t schedule) {
   if (schedule != PT_SCHEDULE_MEGAKERNEL && schedule != PT_SCHEDULE_WAVEFRONT)
     return fail(ctx, PT_ERR_INVALID_ARG, "unknown schedule");
   ctx->schedule = schedule;
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 
 pt_status pt_set_wave_slots(pt_context *ctx, uint32_t slots) {
   if (!ctx || slots == 0) return fail(ctx, PT_ERR_INVALID_ARG, "bad argument");
   ctx->wave_slots = slots;
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 
@@ -1377,6 +1407,7 @@ pt_status pt_debug_fail_allocations(pt_context *ctx, uint32_t count) {
 pt_status pt_set_wave_graphs(pt_context *ctx, int on) {
   if (!ctx) return fail(ctx, PT_ERR_INVALID_ARG, "context is NULL");
   ctx->use_graphs = on != 0;
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 
@@ -1386,6 +1417,7 @@ pt_status pt_set_wave_overlap(pt_context *ctx, int on) {
   ctx->overlap_arenas = on == 0 ? 0u : (on == 1 ? 3u : (uint32_t)on);
   ctx->overlap_waves = ctx->overlap_arenas >= 2;
   ctx->overlap_fixed = on >= 2;
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 
@@ -1393,6 +1425,7 @@ pt_status pt_set_shade_blocks(pt_context *ctx, uint32_t blocks_per_sm) {
   if (!ctx || (blocks_per_sm != 3 && blocks_per_sm != 4))
     return fail(ctx, PT_ERR_INVALID_ARG, "shade blocks per SM must be 3 or 4");
   ctx->shade_blocks = blocks_per_sm;
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 
@@ -1401,12 +1434,14 @@ pt_status pt_set_traversal(pt_context *ctx, uint32_t threads, uint32_t claim_chu
     return fail(ctx, PT_ERR_INVALID_ARG, "traversal threads must be 128 or 256 and the claim chunk 1, 2 or 4");
   ctx->trav_threads = threads;
   ctx->claim_chunk = claim_chunk;
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 
 pt_status pt_set_material_sort(pt_context *ctx, int on) {
   if (!ctx) return fail(ctx, PT_ERR_INVALID_ARG, "context is NULL");
   ctx->material_sort = on != 0;
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 
@@ -1414,6 +1449,7 @@ pt_status pt_set_node_width(pt_context *ctx, uint32_t extension_width, uint32_t 
   if (!ctx || (extension_width != 2 && extension_width != 4) || (shadow_width != 2 && shadow_width != 4))
     return fail(ctx, PT_ERR_INVALID_ARG, "node widths must be 2 or 4");
   ctx->wide_nodes = (extension_width == 4 ? WIDE_EXTENSION : 0u) | (shadow_width == 4 ? WIDE_SHADOW : 0u);
+  ctx->schedule_fixed = true;
   return PT_OK;
 }
 

@@ -36,6 +36,9 @@ struct pt_context {
   // The wavefront is the default schedule (C1: 646 M samples/s against
   // about 200 M for the megakernel); pt_set_schedule / tuned choices change it.
   uint32_t schedule = PT_SCHEDULE_WAVEFRONT;
+  // The schedule (or any setting of the wavefront) was chosen, by a call or
+  // by the tuner: small refines keep it.
+  bool schedule_fixed = false;
   // Path slots per wave. 8 M measured best with overlapped waves (C1: 646 M
   // samples/s against 613 M at 4 M and 474 M at 1 M, three in flight).
   uint32_t wave_slots = 1u << 23;

@@ -146,7 +146,7 @@ PT_DEV bool trace_extension(const DevRequest &rq, const PathState &ps, Hit &hit,
   AcceptFilter acc{&s, &ps.smp, ps.k << 16, ps.k == 0, 0xffffffffu};
   TraversalStats st{0, 0};
   ts.ext_rays++;
-  bool found = closest_hit(s, ps.o, ps.d, 0.0f, inf(), acc, hit, st, ts.err);
+  bool found = closest_hit<false>(s, ps.o, ps.d, 0.0f, inf(), acc, hit, st, ts.err);
   ts.ext_nodes += st.nodes;
   ts.ext_tris += st.tris;
   return found;
@@ -157,7 +157,7 @@ PT_DEV bool trace_shadow(const DevRequest &rq, const PathState &ps, const Shadow
   AcceptFilter acc{&s, &ps.smp, sr.ray_id, false, sr.skip};
   TraversalStats st{0, 0};
   ts.shadow_rays++;
-  bool occ = occluded(s, sr.o, sr.d, 0.0f, sr.tmax, acc, st, ts.err);
+  bool occ = occluded<false>(s, sr.o, sr.d, 0.0f, sr.tmax, acc, st, ts.err);
   ts.sh_nodes += st.nodes;
   ts.sh_tris += st.tris;
   return !occ;

@@ -18,7 +18,9 @@
 
 namespace ptd {
 
-constexpr int kStackSize = 64;  // the host builder caps tree depth below this
+// A four-child node pushes at most three entries per level and the builders
+// keep the binary tree (hence the four-child tree) at most 56 levels deep.
+constexpr int kTravStackSize = 3 * 56 + 8;
 constexpr uint32_t kLeafCountShift = 27;
 constexpr uint32_t kLeafFirstMask = (1u << kLeafCountShift) - 1u;
 
@@ -126,136 +128,223 @@ PT_DEV void node_boxes(const BvhNode *node, const Ray &r, float t0, float t1, bo
   }
 }
 
+// One quantised plane of Bvh4Node: 1 + q / 32768 for byte i of `word`.
+PT_DEV float plane_at(uint32_t word, int i) {
+  return __uint_as_float(__byte_perm(word, 0x3f800000u, 0x7604u + ((uint32_t)i << 4)));
+}
+// The largest / smallest of three; NaN operands are passed over.
+PT_DEV float max3f(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+PT_DEV float min3f(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+PT_DEV int child_of(const int4 &c, uint32_t key) {
+  const int a = (key & 1u) ? c.y : c.x, b = (key & 1u) ? c.w : c.z;
+  return (key & 2u) ? b : a;
+}
+
+// Where the ray meets a node's grid on one axis: plane f = 1 + q / 32768
+// lies at t = step * f + near (or far), the offsets moved apart by the
+// rounding of (base - o) * inv (twice 2^-24 of it) and of the triangle
+// test's own translation by the origin, with room to spare: 2^-21 of a value
+// that is at least 32,768 quanta or the distance to the node.
+struct AxisPlanes {
+  float step, off_near, off_far;
+  uint32_t near_word, far_word;
+  PT_DEV AxisPlanes(float base, float grid, uint32_t lo, uint32_t hi, float o, float inv) {
+    const float slack = 4.76837158e-7f;
+    const float a = (base - o) * inv;
+    step = grid * inv;
+    off_near = fmaf(fabsf(a), -slack, a);
+    off_far = fmaf(fabsf(a), slack, a);
+    near_word = inv < 0.0f ? hi : lo;
+    far_word = inv < 0.0f ? lo : hi;
+  }
+};
+
+// Both planes of child i on one axis by one packed multiply-add (each half
+// rounds as fmaf does).
+PT_DEV void near_far(const AxisPlanes &a, int i, float &n, float &f) {
+  unsigned long long p, st, off, r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(plane_at(a.near_word, i)), "f"(plane_at(a.far_word, i)));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(st) : "f"(a.step));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(off) : "f"(a.off_near), "f"(a.off_far));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(p), "l"(st), "l"(off));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(n), "=f"(f) : "l"(r));
+}
+// The hit children's sort keys: the entry distance's bits with the child
+// index in the low two (which child of two almost equally near ones comes
+// first decides nothing), all ones for a child the ray misses. A box counts
+// as hit when the ray enters it before it leaves it or t_far, either of them
+// widened by 2^-20 for the relative rounding of the plane distances and of a
+// candidate's own t. Rays start at t = 0. An unused slot is an empty leaf
+// with inverted planes: it needs no test of its own and does no harm where
+// its planes round together.
+PT_DEV uint32_t child_key(const AxisPlanes &x, const AxisPlanes &y, const AxisPlanes &z, int i, float t_far) {
+  float nx, ny, nz, fx, fy, fz;
+  near_far(x, i, nx, fx);
+  near_far(y, i, ny, fy);
+  near_far(z, i, nz, fz);
+  const float tn = max3f(nx, ny, fmaxf(nz, 0.0f));
+  const float tf = min3f(fx, fy, fminf(fz, t_far)) * 1.00000095f;
+  return tn <= tf ? (__float_as_uint(tn) & ~3u) | (uint32_t)i : 0xffffffffu;
+}
+
+// One visit of a four-child node: the sort keys of its hit children, nearest
+// first (kNone from the first miss on).
+struct NodeVisit4 {
+  static constexpr uint32_t kNone = 0xffffffffu;
+  int4 child;
+  uint32_t first, second, third, last;
+  PT_DEV NodeVisit4(const Bvh4Node *nd, V3 o, V3 inv, float t_far) {
+    const float4 base = ldg4(&nd->base);
+    const uint4 mid = __ldg(&nd->mid), pl = __ldg(&nd->planes);
+    child = __ldg(&nd->child);
+    const AxisPlanes x(base.x, base.w, mid.z, mid.w, o.x, inv.x);
+    const AxisPlanes y(base.y, __uint_as_float(mid.x), pl.x, pl.y, o.y, inv.y);
+    const AxisPlanes z(base.z, __uint_as_float(mid.y), pl.z, pl.w, o.z, inv.z);
+    const uint32_t k0 = child_key(x, y, z, 0, t_far), k1 = child_key(x, y, z, 1, t_far);
+    const uint32_t k2 = child_key(x, y, z, 2, t_far), k3 = child_key(x, y, z, 3, t_far);
+    const uint32_t a = min(k0, k1), b = max(k0, k1), c = min(k2, k3), d = max(k2, k3);
+    const uint32_t m0 = max(a, c), m1 = min(b, d);
+    first = min(a, c);
+    last = max(b, d);
+    second = min(m0, m1);
+    third = max(m0, m1);
+  }
+  PT_DEV int ref(uint32_t key) const { return child_of(child, key); }
+};
+
 struct TraversalStats {
   uint32_t nodes, tris;
 };
 
-// Closest accepted hit in [t_min, t_max]. `accept(g, t, b0, b1, b2, front)`
-// is the any-hit filter (alpha mask, stochastic blend, primary culling).
-template <class Accept>
-PT_DEV bool closest_hit(const DevScene &s, V3 o, V3 d, float t_min, float t_max, Accept &&accept, Hit &best,
-                        TraversalStats &st, uint32_t &err) {
-  if (s.node_count == 0) return false;
-  Ray r = make_ray(o, d);
-  bool have = false;
-  best.t = t_max;
-  best.g = 0xffffffffu;
-  int stack[kStackSize];
-  int sp = 0;
-  int cur = 0;
+// One thread's walk of the tree, in its four-child (kWide) or two-child
+// layout: `leaf(first, count)` for every leaf whose box the ray meets before
+// `t_far()`, nearest boxes first; ends when it returns true.
+template <bool kWide, class Far, class Leaf>
+PT_DEV void walk_tree(const DevScene &s, const Ray &r, TraversalStats &st, uint32_t &err, Far &&t_far, Leaf &&leaf) {
+  if (s.node_count == 0) return;
+  constexpr int kStack = kWide ? kTravStackSize : 64;
+  int stack[kStack];
+  int sp = 0, cur = 0;
   for (;;) {
     if (cur >= 0) {
       st.nodes++;
-      bool h0, h1;
-      float e0, e1;
-      int4 dd;
-      node_boxes(s.nodes + cur, r, t_min, best.t, h0, h1, e0, e1, dd);
-      if (h0 && h1) {
-        int nearc = e1 < e0 ? dd.y : dd.x;
-        int farc = e1 < e0 ? dd.x : dd.y;
-        if (sp < kStackSize) {
-          stack[sp++] = farc;
-        } else {
-          err |= ERR_STACK_OVERFLOW;
+      if constexpr (kWide) {
+        const NodeVisit4 nv(s.nodes4 + cur, r.o, r.inv, t_far());
+        if (nv.first != NodeVisit4::kNone) {
+          if (sp + 3 > kStack) {
+            err |= ERR_STACK_OVERFLOW;
+          } else {
+            if (nv.last != NodeVisit4::kNone) stack[sp++] = nv.ref(nv.last);
+            if (nv.third != NodeVisit4::kNone) stack[sp++] = nv.ref(nv.third);
+            if (nv.second != NodeVisit4::kNone) stack[sp++] = nv.ref(nv.second);
+          }
+          cur = nv.ref(nv.first);
+          continue;
         }
-        cur = nearc;
-        continue;
-      }
-      if (h0) {
-        cur = dd.x;
-        continue;
-      }
-      if (h1) {
-        cur = dd.y;
-        continue;
+      } else {
+        bool h0, h1;
+        float e0, e1;
+        int4 dd;
+        node_boxes(s.nodes + cur, r, 0.0f, t_far(), h0, h1, e0, e1, dd);
+        if (h0 && h1) {
+          const bool swap = e1 < e0;
+          if (sp + 1 > kStack)
+            err |= ERR_STACK_OVERFLOW;
+          else
+            stack[sp++] = swap ? dd.x : dd.y;
+          cur = swap ? dd.y : dd.x;
+          continue;
+        }
+        if (h0 || h1) {
+          cur = h0 ? dd.x : dd.y;
+          continue;
+        }
       }
     } else {
       // Leaf reference ~(first | count << 27): records [first, first + count).
-      uint32_t first = (uint32_t)(~cur);
-      uint32_t count = first >> kLeafCountShift;
-      first &= kLeafFirstMask;
-      for (uint32_t i = 0; i < count; ++i) {
-        const float4 *tr = s.tris + 3u * (first + i);
-        float4 p0 = ldg4(tr), p1 = ldg4(tr + 1), p2 = ldg4(tr + 2);
-        st.tris++;
-        float t, b0, b1, b2;
-        bool front;
-        if (!intersect_watertight(r, {p0.x, p0.y, p0.z}, {p1.x, p1.y, p1.z}, {p2.x, p2.y, p2.z}, t, b0, b1, b2, front))
-          continue;
-        if (!(t >= t_min)) continue;
-        uint32_t g = __float_as_uint(p0.w);
-        bool better = have ? (t < best.t || (t == best.t && g < best.g)) : (t <= t_max);
-        if (!better) continue;
-        if (accept(g, __float_as_uint(p1.w), t, b0, b1, b2, front)) {
-          best.t = t;
-          best.g = g;
-          best.b0 = b0;
-          best.b1 = b1;
-          best.b2 = b2;
-          best.front = front;
-          have = true;
-        }
-      }
+      const uint32_t range = (uint32_t)(~cur);
+      if (leaf(range & kLeafFirstMask, range >> kLeafCountShift)) return;
     }
-    if (sp == 0) break;
+    if (sp == 0) return;
     cur = stack[--sp];
   }
+}
+
+// Closest accepted hit in [t_min, t_max] (t_min >= 0). `accept(g, t, b0, b1, b2, front)`
+// is the any-hit filter (alpha mask, stochastic blend, primary culling).
+template <bool kWide = true, class Accept>
+PT_DEV bool closest_hit(const DevScene &s, V3 o, V3 d, float t_min, float t_max, Accept &&accept, Hit &best,
+                        TraversalStats &st, uint32_t &err) {
+  const Ray r = make_ray(o, d);
+  bool have = false;
+  best.t = t_max;
+  best.g = 0xffffffffu;
+  walk_tree<kWide>(
+      s, r, st, err, [&] { return best.t; },
+      [&](uint32_t first, uint32_t count) {
+        for (uint32_t i = 0; i < count; ++i) {
+          const float4 *tr = s.tris + 3u * (first + i);
+          const float4 p0 = ldg4(tr), p1 = ldg4(tr + 1), p2 = ldg4(tr + 2);
+          st.tris++;
+          float t, b0, b1, b2;
+          bool front;
+          if (!intersect_watertight(r, {p0.x, p0.y, p0.z}, {p1.x, p1.y, p1.z}, {p2.x, p2.y, p2.z}, t, b0, b1, b2,
+                                    front))
+            continue;
+          if (!(t >= t_min)) continue;
+          const uint32_t g = __float_as_uint(p0.w);
+          const bool better = have ? (t < best.t || (t == best.t && g < best.g)) : (t <= t_max);
+          if (!better) continue;
+          if (accept(g, __float_as_uint(p1.w), t, b0, b1, b2, front)) {
+            best.t = t;
+            best.g = g;
+            best.b0 = b0;
+            best.b1 = b1;
+            best.b2 = b2;
+            best.front = front;
+            have = true;
+          }
+        }
+        return false;
+      });
   return have;
 }
 
 // Any accepted hit in [t_min, t_max].
-template <class Accept>
+template <bool kWide = true, class Accept>
 PT_DEV bool occluded(const DevScene &s, V3 o, V3 d, float t_min, float t_max, Accept &&accept, TraversalStats &st,
                      uint32_t &err) {
-  if (s.node_count == 0) return false;
-  Ray r = make_ray(o, d);
-  int stack[kStackSize];
-  int sp = 0;
-  int cur = 0;
-  for (;;) {
-    if (cur >= 0) {
-      st.nodes++;
-      bool h0, h1;
-      float e0, e1;
-      int4 dd;
-      node_boxes(s.nodes + cur, r, t_min, t_max, h0, h1, e0, e1, dd);
-      if (h0 && h1) {
-        if (sp < kStackSize) {
-          stack[sp++] = dd.y;
-        } else {
-          err |= ERR_STACK_OVERFLOW;
+  const Ray r = make_ray(o, d);
+  bool hit = false;
+  walk_tree<kWide>(
+      s, r, st, err, [&] { return t_max; },
+      [&](uint32_t first, uint32_t count) {
+        for (uint32_t i = 0; i < count; ++i) {
+          const float4 *tr = s.tris + 3u * (first + i);
+          const float4 p0 = ldg4(tr), p1 = ldg4(tr + 1), p2 = ldg4(tr + 2);
+          st.tris++;
+          float t, b0, b1, b2;
+          bool front;
+          if (!intersect_watertight(r, {p0.x, p0.y, p0.z}, {p1.x, p1.y, p1.z}, {p2.x, p2.y, p2.z}, t, b0, b1, b2,
+                                    front))
+            continue;
+          if (!(t >= t_min && t <= t_max)) continue;
+          if (accept(__float_as_uint(p0.w), __float_as_uint(p1.w), t, b0, b1, b2, front)) {
+            hit = true;
+            return true;
+          }
         }
-        cur = dd.x;
-        continue;
-      }
-      if (h0) {
-        cur = dd.x;
-        continue;
-      }
-      if (h1) {
-        cur = dd.y;
-        continue;
-      }
-    } else {
-      uint32_t first = (uint32_t)(~cur);
-      uint32_t count = first >> kLeafCountShift;
-      first &= kLeafFirstMask;
-      for (uint32_t i = 0; i < count; ++i) {
-        const float4 *tr = s.tris + 3u * (first + i);
-        float4 p0 = ldg4(tr), p1 = ldg4(tr + 1), p2 = ldg4(tr + 2);
-        st.tris++;
-        float t, b0, b1, b2;
-        bool front;
-        if (!intersect_watertight(r, {p0.x, p0.y, p0.z}, {p1.x, p1.y, p1.z}, {p2.x, p2.y, p2.z}, t, b0, b1, b2, front))
-          continue;
-        if (!(t >= t_min && t <= t_max)) continue;
-        if (accept(__float_as_uint(p0.w), __float_as_uint(p1.w), t, b0, b1, b2, front)) return true;
-      }
-    }
-    if (sp == 0) break;
-    cur = stack[--sp];
-  }
-  return false;
+        return false;
+      });
+  return hit;
 }
 
 // ---------------------------------------------------------------- attributes

@@ -36,9 +36,6 @@ namespace ptd {
 // 62.9 / 64.0 / 63.6 ms, sphere grid 49.5 / 48.7 / 48.6 / 49.1 / 49.2 ms.
 constexpr int kShortStack = 16;
 constexpr int kTravDone = (int)0x80000000;  // "no next node": neither a node index nor a leaf reference
-// A four-child node pushes at most three entries per level and the builder
-// keeps the binary tree (hence the four-child tree) at most 56 levels deep.
-constexpr int kTravStackSize = 3 * 56 + 8;
 // Rows of a block's shared words, one word per thread each: the stack, then
 // the thread's node visits, triangle tests and rays.
 enum TravRows : int { ROW_NODES = kShortStack, ROW_TRIS, ROW_RAYS, ROW_COUNT };
@@ -103,73 +100,6 @@ struct TravStack {
   }
 };
 
-// One quantised plane of Bvh4Node: 1 + q / 32768 for byte i of `word`.
-PT_DEV float plane_at(uint32_t word, int i) {
-  return __uint_as_float(__byte_perm(word, 0x3f800000u, 0x7604u + ((uint32_t)i << 4)));
-}
-// The largest / smallest of three; NaN operands are passed over.
-PT_DEV float max3f(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-PT_DEV float min3f(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-PT_DEV int child_of(const int4 &c, uint32_t key) {
-  const int a = (key & 1u) ? c.y : c.x, b = (key & 1u) ? c.w : c.z;
-  return (key & 2u) ? b : a;
-}
-
-// Where the ray meets a node's grid on one axis: plane f = 1 + q / 32768
-// lies at t = step * f + near (or far), the offsets moved apart by the
-// rounding of (base - o) * inv (twice 2^-24 of it) and of the triangle
-// test's own translation by the origin, with room to spare: 2^-21 of a value
-// that is at least 32,768 quanta or the distance to the node.
-struct AxisPlanes {
-  float step, off_near, off_far;
-  uint32_t near_word, far_word;
-  PT_DEV AxisPlanes(float base, float grid, uint32_t lo, uint32_t hi, float o, float inv) {
-    const float slack = 4.76837158e-7f;
-    const float a = (base - o) * inv;
-    step = grid * inv;
-    off_near = fmaf(fabsf(a), -slack, a);
-    off_far = fmaf(fabsf(a), slack, a);
-    near_word = inv < 0.0f ? hi : lo;
-    far_word = inv < 0.0f ? lo : hi;
-  }
-};
-
-// Both planes of child i on one axis by one packed multiply-add (each half
-// rounds as fmaf does).
-PT_DEV void near_far(const AxisPlanes &a, int i, float &n, float &f) {
-  unsigned long long p, st, off, r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(plane_at(a.near_word, i)), "f"(plane_at(a.far_word, i)));
-  asm("mov.b64 %0, {%1, %1};" : "=l"(st) : "f"(a.step));
-  asm("mov.b64 %0, {%1, %2};" : "=l"(off) : "f"(a.off_near), "f"(a.off_far));
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(p), "l"(st), "l"(off));
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(n), "=f"(f) : "l"(r));
-}
-// The hit children's sort keys: the entry distance's bits with the child
-// index in the low two (which child of two almost equally near ones comes
-// first decides nothing), all ones for a child the ray misses. A box counts
-// as hit when the ray enters it before it leaves it or t_far, either of them
-// widened by 2^-20 for the relative rounding of the plane distances and of a
-// candidate's own t. Rays start at t = 0. An unused slot is an empty leaf
-// with inverted planes: it needs no test of its own and does no harm where
-// its planes round together.
-PT_DEV uint32_t child_key(const AxisPlanes &x, const AxisPlanes &y, const AxisPlanes &z, int i, float t_far) {
-  float nx, ny, nz, fx, fy, fz;
-  near_far(x, i, nx, fx);
-  near_far(y, i, ny, fy);
-  near_far(z, i, nz, fz);
-  const float tn = max3f(nx, ny, fmaxf(nz, 0.0f));
-  const float tf = min3f(fx, fy, fminf(fz, t_far)) * 1.00000095f;
-  return tn <= tf ? (__float_as_uint(tn) & ~3u) | (uint32_t)i : 0xffffffffu;
-}
-
 // Traversal state of one ray. `cur` is the next node (>= 0), a leaf that
 // waits for the parked one (< 0) or kTravDone; `leaf` the parked leaf's
 // records still to test (first | count << kLeafCountShift). A leaf waits in
@@ -229,18 +159,9 @@ struct TravCore {
     stk.count(words, ROW_NODES);
     if (kOnly4 || wide) {
       const Bvh4Node *nd = nodes4 + cur;
-      const float4 base = ldg4(&nd->base);
-      const uint4 mid = __ldg(&nd->mid), pl = __ldg(&nd->planes);
-      const int4 ch = __ldg(&nd->child);
-      const AxisPlanes x(base.x, base.w, mid.z, mid.w, o.x, inv.x);
-      const AxisPlanes y(base.y, __uint_as_float(mid.x), pl.x, pl.y, o.y, inv.y);
-      const AxisPlanes z(base.z, __uint_as_float(mid.y), pl.z, pl.w, o.z, inv.z);
-      const uint32_t none = 0xffffffffu;
-      const uint32_t k0 = child_key(x, y, z, 0, t_far), k1 = child_key(x, y, z, 1, t_far);
-      const uint32_t k2 = child_key(x, y, z, 2, t_far), k3 = child_key(x, y, z, 3, t_far);
-      const uint32_t a = min(k0, k1), b = max(k0, k1), c = min(k2, k3), d = max(k2, k3);
-      const uint32_t first = min(a, c), m0 = max(a, c), m1 = min(b, d), last = max(b, d);
-      const uint32_t second = min(m0, m1), third = max(m0, m1);
+      const NodeVisit4 nv(nd, o, inv, t_far);
+      const int4 &ch = nv.child;
+      const uint32_t none = NodeVisit4::kNone, first = nv.first, second = nv.second, third = nv.third, last = nv.last;
       if (stk.room_for_three(words)) {
         // Everything below stays in shared memory: no branches but the last.
         if (third != none) {

@@ -2,7 +2,9 @@
 
 Renders the 36-triangle Cornell box at 32x32 / 8 spp through the C ABI and
 requires (a) bit-exact camera-ray hits and (b) HDR parity (MAE <= 2e-3,
-PSNR >= 45 dB) against the CPU restatement. Raises on any mismatch.
+PSNR >= 45 dB) against the CPU restatement, and (c) the same accumulator from
+the wavefront and from what the library picks for so small a call. Raises on
+any mismatch.
 """
 from __future__ import annotations
 
@@ -12,7 +14,7 @@ import numpy as np
 
 
 def run() -> None:
-    from . import api, testscenes as ts
+    from . import abi, api, testscenes as ts
     from .options import PathTraceOptions
     from .scene import Camera
 
@@ -44,5 +46,12 @@ def run() -> None:
     ext, shadow = t.ray_counts()
     print(f"smoke ok: MAE {mae:.2e} PSNR {psnr:.1f} dB, {ext} extension + {shadow} shadow rays, "
           f"{t.last_kernel_ms():.3f} ms")
+    ctx.set_schedule(abi.PT_SCHEDULE_WAVEFRONT)
+    w = api.PathTracer(ctx)
+    w.sync(scene, opts)
+    w.refine(8)
+    if not np.array_equal(w.accum(), t.accum()):
+        raise AssertionError("the wavefront's accumulator differs")
+    w.close()
     t.close()
     ctx.close()

@@ -1,7 +1,9 @@
-"""Wavefront traversal (quantised four-child nodes, voted steps) against the
-megakernel's two-child traversal: the accumulators are equal bit for bit for
-geometry of any size, place and distance from the camera, for rays along the
-axes, for deep stacks and for queues smaller than a warp."""
+"""Traversal of the quantised four-child nodes (the wavefront's voted steps,
+and the raycast backend's walk in its own tests) against the two-child nodes,
+whose boxes are full precision, in the wavefront and in the megakernel: the
+accumulators are equal bit for bit for geometry of any size, place and
+distance from the camera, for rays along the axes, for deep stacks and for
+queues smaller than a warp."""
 import copy
 import math
 
@@ -28,9 +30,14 @@ def placed_soup(tris, scale, offset, distance):
 
 
 def both(ctx, scene, opts):
+    """(accumulator, ray counts) with the four-child nodes, then with the
+    two-child ones; the megakernel (two-child nodes, one thread a path) must
+    agree with them."""
     out = []
-    for schedule in (abi.PT_SCHEDULE_WAVEFRONT, abi.PT_SCHEDULE_MEGAKERNEL):
+    for schedule, width in ((abi.PT_SCHEDULE_WAVEFRONT, 4), (abi.PT_SCHEDULE_WAVEFRONT, 2),
+                            (abi.PT_SCHEDULE_MEGAKERNEL, 4)):
         ctx.set_schedule(schedule)
+        ctx.set_node_width(width, width)
         try:
             t = api.PathTracer(ctx)
             t.sync(scene, opts)
@@ -39,7 +46,9 @@ def both(ctx, scene, opts):
             t.close()
         finally:
             ctx.set_schedule(abi.PT_SCHEDULE_WAVEFRONT)
-    return out
+            ctx.set_node_width(4, 4)
+    assert np.array_equal(out[0][0], out[2][0], equal_nan=True) and out[0][1] == out[2][1]
+    return out[:2]
 
 
 @pytest.mark.parametrize("scale,offset,distance", [(1.0, 0.0, 1.0), (1e-3, 0.0, 600.0), (1e4, -3e4, 0.1),
