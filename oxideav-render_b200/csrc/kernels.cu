@@ -318,8 +318,7 @@ cudaError_t launch_wavefront(const WaveBuffers &w, DevCounters *ctr, int num_sms
   if (e == cudaSuccess && w.sort_materials)
     e = cudaMemsetAsync(w.sort_counts, 0, sizeof(uint32_t) * 2 * kSortBuckets * (w.iterations + 1), st);
   if (e != cudaSuccess) return e;
-  const uint32_t g_sort = (uint32_t)num_sms * 6, g_wide = (uint32_t)num_sms * 16,
-                 g_nee = (uint32_t)num_sms * 8;
+  const uint32_t g_sort = (uint32_t)num_sms * 6, g_wide = (uint32_t)num_sms * 16;
   tm.mark(STAGE_RAYGEN, st);
   k_wf_raygen<<<g_wide, 256, 0, st>>>(w);
   for (uint32_t it = 0; it < w.iterations; ++it) {
@@ -332,7 +331,7 @@ cudaError_t launch_wavefront(const WaveBuffers &w, DevCounters *ctr, int num_sms
       k_wf_sort_scatter<<<g_sort, 256, 0, st>>>(w, it);
     }
     tm.mark(STAGE_NEE, st);
-    k_wf_nee<<<g_nee, 256, 0, st>>>(w, it);
+    k_wf_nee<<<num_sms * kNeeBlocks * 2, kNeeThreads, 0, st>>>(w, it);
     tm.mark(STAGE_SHADE, st);
     if (w.sort_materials) launch_wf_shade_plain(w, it, num_sms, st);
     if (w.layered || !w.sort_materials) {

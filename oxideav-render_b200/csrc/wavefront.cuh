@@ -161,16 +161,21 @@ __global__ void __launch_bounds__(256) k_wf_sort_scatter(WaveBuffers w, uint32_t
 // The area-light sample and emission MIS pdf of every queued vertex that
 // hit something, in the order shade will read them (its queue). Values are
 // those shade would compute inline (the same functions on the same inputs).
-// Four blocks of 256 per SM (64 registers, a few spills): the sampling is
-// latency bound (CDF searches, dependent f64 steps), so occupancy beats the
-// spill-free 106-register form (NEE stage 128 -> 120 ms per mix step).
-__global__ void __launch_bounds__(256, 4) k_wf_nee(WaveBuffers w, uint32_t iter) {
+// 1,024 threads per SM (64 registers, a few spills): the sampling is latency
+// bound (CDF searches, dependent f64 steps), so occupancy beats the
+// spill-free 106-register form (Cornell box 1.95 ms a frame at 512 threads,
+// 1.74 at 768). The barrier keeps a block's warps on the same code, as in
+// k_wf_shade: blocks of 256 without it 1.73, with it 1.65, of 512 1.60
+// (stress scene 11.85 / 11.54 / 11.12).
+constexpr int kNeeThreads = 512, kNeeBlocks = 2;
+__global__ void __launch_bounds__(kNeeThreads, kNeeBlocks) k_wf_nee(WaveBuffers w, uint32_t iter) {
   if (!(w.desc->flags & WAVE_AREA_LIGHTS)) return;  // nothing to sample in this wave
   const DevRequest *reqs = w.desc->reqs;
   const uint32_t n = w.counters[iter * kWfCounterStride + 0];
   const uint32_t *q = w.sort_materials ? w.q_sorted : w.q[iter & 1u];
   const size_t cap = w.capacity;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; __syncthreads_or(i < n); i += gridDim.x * blockDim.x) {
+    if (i >= n) continue;
     const uint32_t slot = q[i];
     const uint32_t hg = w.hit_g[slot];
     if (!(hg & HIT_FOUND)) continue;
