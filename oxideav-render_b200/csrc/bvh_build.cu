@@ -601,6 +601,7 @@ __global__ void k_write_records(Nodes nd, const uint32_t *vals, const float *pos
 constexpr int kSahBins = 16;
 constexpr uint32_t kSahNone = 0xffffffffu;
 constexpr uint32_t kSahHalve = 0xfffffffeu;
+constexpr uint32_t kSahBinTile = kThreads * 4;
 constexpr int kSahBinWords = 3 * kSahBins * 7;  // per axis and bin: count, lo.xyz, hi.xyz
 
 struct SahNodes {
@@ -701,13 +702,37 @@ __device__ __forceinline__ void node_binning(const uint32_t *b, float clo[3], fl
   }
 }
 
+// One triangle into the bins of its node, `kShared` in the block's shared
+// memory. There most triangles extend no bound: the read before each minimum
+// and maximum is a broadcast where the atomics of a warp, which fall into few
+// bins, would queue.
+template <bool kShared>
+__device__ __forceinline__ void sah_add_bins(uint32_t *dst, const float l[3], const float h[3], const float c[3],
+                                             const float clo[3], const float scale[3], const bool use[3]) {
+  uint32_t ol[3], oh[3];
+  for (int q = 0; q < 3; ++q) {
+    ol[q] = ord_of(l[q]);
+    oh[q] = ord_of(h[q]);
+  }
+  for (int k = 0; k < 3; ++k) {
+    if (!use[k]) continue;
+    uint32_t *w = dst + (k * kSahBins + sah_bin((c[k] - clo[k]) * scale[k])) * 7;
+    atomicAdd(w, 1u);
+    for (int q = 0; q < 3; ++q) {
+      if (!kShared || ol[q] < w[1 + q]) atomicMin(w + 1 + q, ol[q]);
+      if (!kShared || oh[q] > w[4 + q]) atomicMax(w + 4 + q, oh[q]);
+    }
+  }
+}
+
 // Bin counts and bounds: a tile of triangles of one node accumulates in
 // shared memory and flushes once; tiles spanning several nodes (small
-// nodes) update the nodes' bins directly.
+// nodes) update the nodes' bins directly. Tiles of 1,024 triangles: 200k of
+// them are 196 blocks, more than one an SM (2,048 left a third of them idle).
 __global__ void __launch_bounds__(kThreads) k_sah_bins(const float4 *plo, const float4 *phi, const uint32_t *seg,
                                                        uint32_t n, SahLevel lv) {
   __shared__ uint32_t sb[kSahBinWords];
-  constexpr uint32_t kTile = kThreads * 8;
+  constexpr uint32_t kTile = kSahBinTile;
   for (uint32_t t0 = blockIdx.x * kTile; t0 < n; t0 += gridDim.x * kTile) {
     const uint32_t t1 = min(n, t0 + kTile);
     const uint32_t sa = seg[t0], sz = seg[t1 - 1];
@@ -727,17 +752,10 @@ __global__ void __launch_bounds__(kThreads) k_sah_bins(const float4 *plo, const 
       node_binning(lv.bnd + 12ull * s, clo, scale, use);
       float l[3], h[3], c[3];
       prim_box(plo, phi, i, l, h, c);
-      uint32_t *dst = uniform ? sb : lv.bins + (uint64_t)kSahBinWords * s;
-      for (int k = 0; k < 3; ++k) {
-        if (!use[k]) continue;
-        const int bin = sah_bin((c[k] - clo[k]) * scale[k]);
-        uint32_t *w = dst + (k * kSahBins + bin) * 7;
-        atomicAdd(w, 1u);
-        for (int a = 0; a < 3; ++a) {
-          atomicMin(w + 1 + a, ord_of(l[a]));
-          atomicMax(w + 4 + a, ord_of(h[a]));
-        }
-      }
+      if (uniform)
+        sah_add_bins<true>(sb, l, h, c, clo, scale, use);
+      else
+        sah_add_bins<false>(lv.bins + (uint64_t)kSahBinWords * s, l, h, c, clo, scale, use);
     }
     if (uniform) {
       __syncthreads();
@@ -770,82 +788,116 @@ __global__ void k_sah_init_bins(SahLevel lv) {
   }
 }
 
-// The split of every active node (the host builder's sweep).
+// The cheapest split over a node's bins (the host builder's sweep), by a
+// warp: a half-warp per axis, a lane per bin, the running boxes from both
+// ends by shuffles (minimum, maximum and count are exact in any order), a
+// lane per split plane, and the first of the cheapest in the host's order
+// (axis, then plane). Returns axis << 8 | plane in every lane, or kSahNone
+// when no plane has triangles on both sides. One thread per node took 48 us a
+// level whatever the level's size, most of it local-memory arrays.
+__device__ uint32_t sah_best_split(const uint32_t *bins, const bool use[3], float parent, float &best_cost) {
+  const uint32_t lane = threadIdx.x & 31u;
+  float best = INFINITY;
+  uint32_t best_at = kSahNone;
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const int k = 2 * pass + (int)(lane >> 4), bb = (int)(lane & 15u);
+    const bool on = k < 3 && (k == 0 ? use[0] : (k == 1 ? use[1] : use[2]));
+    float ll[3], lh[3], rl[3], rh[3];
+    uint32_t lc = 0;
+    for (int q = 0; q < 3; ++q) {
+      ll[q] = INFINITY;
+      lh[q] = -INFINITY;
+    }
+    if (on) {
+      const uint32_t *w = bins + (k * kSahBins + bb) * 7;
+      lc = w[0];
+      if (lc)
+        for (int q = 0; q < 3; ++q) {
+          ll[q] = float_of(w[1 + q]);
+          lh[q] = float_of(w[4 + q]);
+        }
+    }
+    uint32_t rc = lc;
+    for (int q = 0; q < 3; ++q) {
+      rl[q] = ll[q];
+      rh[q] = lh[q];
+    }
+    for (int d = 1; d < kSahBins; d <<= 1) {
+      const uint32_t c0 = __shfl_up_sync(0xffffffffu, lc, d, 16), c1 = __shfl_down_sync(0xffffffffu, rc, d, 16);
+      const bool up = bb >= d, down = bb + d < kSahBins;
+      if (up) lc += c0;
+      if (down) rc += c1;
+      for (int q = 0; q < 3; ++q) {
+        const float a0 = __shfl_up_sync(0xffffffffu, ll[q], d, 16), a1 = __shfl_up_sync(0xffffffffu, lh[q], d, 16);
+        const float b0 = __shfl_down_sync(0xffffffffu, rl[q], d, 16), b1 = __shfl_down_sync(0xffffffffu, rh[q], d, 16);
+        if (up) {
+          ll[q] = fminf(ll[q], a0);
+          lh[q] = fmaxf(lh[q], a1);
+        }
+        if (down) {
+          rl[q] = fminf(rl[q], b0);
+          rh[q] = fmaxf(rh[q], b1);
+        }
+      }
+    }
+    // Plane s = bb: bins below it on the left, from it on the right.
+    const uint32_t left = __shfl_up_sync(0xffffffffu, lc, 1, 16);
+    for (int q = 0; q < 3; ++q) {
+      ll[q] = __shfl_up_sync(0xffffffffu, ll[q], 1, 16);
+      lh[q] = __shfl_up_sync(0xffffffffu, lh[q], 1, 16);
+    }
+    if (on && bb >= 1 && left && rc) {
+      const float4 l4 = make_float4(ll[0], ll[1], ll[2], 0.0f), h4 = make_float4(lh[0], lh[1], lh[2], 0.0f);
+      const float4 r4l = make_float4(rl[0], rl[1], rl[2], 0.0f), r4h = make_float4(rh[0], rh[1], rh[2], 0.0f);
+      const float cost =
+          1.0f + (host_area(l4, h4) * (float)left + host_area(r4l, r4h) * (float)rc) / fmaxf(parent, 1e-30f);
+      if (cost < best) {
+        best = cost;
+        best_at = (uint32_t)k << 8 | (uint32_t)bb;
+      }
+    }
+  }
+  for (int d = 16; d > 0; d >>= 1) {
+    const float c = __shfl_xor_sync(0xffffffffu, best, d);
+    const uint32_t at = __shfl_xor_sync(0xffffffffu, best_at, d);
+    if (c < best || (c == best && at < best_at)) {
+      best = c;
+      best_at = at;
+    }
+  }
+  best_cost = best;
+  return best_at;
+}
+
+// The split of every active node, a warp each.
 __global__ void k_sah_split(SahNodes nd, SahLevel lv, uint32_t *max_depth) {
-  for (uint32_t a = blockIdx.x * blockDim.x + threadIdx.x; a < lv.m; a += gridDim.x * blockDim.x) {
+  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * blockDim.x / 32;
+  for (uint32_t a = (blockIdx.x * blockDim.x + threadIdx.x) / 32; a < lv.m; a += warps) {
     const uint32_t v = lv.act[a];
     const uint32_t *b = lv.bnd + 12ull * a;
     const float4 lo = make_float4(float_of(b[0]), float_of(b[1]), float_of(b[2]), 0.0f);
     const float4 hi = make_float4(float_of(b[3]), float_of(b[4]), float_of(b[5]), 0.0f);
-    nd.lo[v] = lo;
-    nd.hi[v] = hi;
     const uint32_t cnt = nd.count[v], depth = nd.depth[v];
-    if (cnt <= 1) {
-      lv.split[a] = kSahNone;
-      atomicMax(max_depth, depth);
-      continue;
-    }
+    uint32_t split = kSahHalve;
     uint32_t need = 0;
     for (uint32_t c = cnt; c > kMaxLeafTris; c = (c + 1) / 2) ++need;
-    const bool median = depth + need >= 56;
-    int axis = -1, best_bin = 0;
-    float best_cost = INFINITY;
-    if (!median) {
-      const float parent = host_area(lo, hi);
+    if (cnt <= 1) {
+      split = kSahNone;
+    } else if (depth + need < 56) {
       bool use[3];
-      float clo[3], scale[3];
+      float clo[3], scale[3], cost;
       node_binning(b, clo, scale, use);
-      const uint32_t *bins = lv.bins + (uint64_t)kSahBinWords * a;
-      for (int k = 0; k < 3; ++k) {
-        if (!use[k]) continue;
-        float rl[kSahBins][3], rh[kSahBins][3];
-        uint32_t rc[kSahBins];
-        float accl[3] = {INFINITY, INFINITY, INFINITY}, acch[3] = {-INFINITY, -INFINITY, -INFINITY};
-        uint32_t acc = 0;
-        for (int bb = kSahBins - 1; bb >= 1; --bb) {
-          const uint32_t *w = bins + (k * kSahBins + bb) * 7;
-          acc += w[0];
-          if (w[0])
-            for (int q = 0; q < 3; ++q) {
-              accl[q] = fminf(accl[q], float_of(w[1 + q]));
-              acch[q] = fmaxf(acch[q], float_of(w[4 + q]));
-            }
-          rc[bb] = acc;
-          for (int q = 0; q < 3; ++q) {
-            rl[bb][q] = accl[q];
-            rh[bb][q] = acch[q];
-          }
-        }
-        float ll[3] = {INFINITY, INFINITY, INFINITY}, lh[3] = {-INFINITY, -INFINITY, -INFINITY};
-        uint32_t lc = 0;
-        for (int s = 1; s < kSahBins; ++s) {
-          const uint32_t *w = bins + (k * kSahBins + s - 1) * 7;
-          lc += w[0];
-          if (w[0])
-            for (int q = 0; q < 3; ++q) {
-              ll[q] = fminf(ll[q], float_of(w[1 + q]));
-              lh[q] = fmaxf(lh[q], float_of(w[4 + q]));
-            }
-          if (lc == 0 || rc[s] == 0) continue;
-          const float4 l4 = make_float4(ll[0], ll[1], ll[2], 0.0f), h4 = make_float4(lh[0], lh[1], lh[2], 0.0f);
-          const float4 r4l = make_float4(rl[s][0], rl[s][1], rl[s][2], 0.0f);
-          const float4 r4h = make_float4(rh[s][0], rh[s][1], rh[s][2], 0.0f);
-          const float cost =
-              1.0f + (host_area(l4, h4) * (float)lc + host_area(r4l, r4h) * (float)rc[s]) / fmaxf(parent, 1e-30f);
-          if (cost < best_cost) {
-            best_cost = cost;
-            axis = k;
-            best_bin = s;
-          }
-        }
-      }
-      if (cnt <= kMaxLeafTris && (axis < 0 || (float)cnt <= best_cost)) {
-        lv.split[a] = kSahNone;
-        atomicMax(max_depth, depth);
-        continue;
-      }
+      const uint32_t at = sah_best_split(lv.bins + (uint64_t)kSahBinWords * a, use, host_area(lo, hi), cost);
+      if (at != kSahNone) split = at;
+      if (cnt <= kMaxLeafTris && (at == kSahNone || (float)cnt <= cost)) split = kSahNone;
     }
-    lv.split[a] = axis >= 0 ? ((uint32_t)axis << 8 | (uint32_t)best_bin) : kSahHalve;
+    if (lane == 0) {
+      nd.lo[v] = lo;
+      nd.hi[v] = hi;
+      lv.split[a] = split;
+      if (split == kSahNone) atomicMax(max_depth, depth);
+    }
   }
 }
 
@@ -1111,146 +1163,122 @@ __global__ void k_sah_small_clear(SahNodes nd, uint32_t v0, uint32_t v1) {
   }
 }
 
-// The whole subtree of one small node, depth first (the host builder's
-// split of a node, sequentially: bounds, 16 bins per axis, the sweep, leaf
-// or split, then an in-place partition).
-__global__ void k_sah_small(const uint32_t *deferred, uint32_t nd_count, const uint32_t *first_id, SahNodes nd,
-                            float4 *plo, float4 *phi, uint32_t *used, uint32_t *max_depth) {
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nd_count; k += gridDim.x * blockDim.x) {
-    const uint32_t root = deferred[k];
-    uint32_t next = first_id[k];
-    const uint32_t id0 = next;
-    struct Task {
-      uint32_t v, b, c, d;
-    } st[2 * kSahSmall];
-    int sp = 0;
-    st[sp++] = {root, nd.begin[root], nd.count[root], nd.depth[root]};
+// The whole subtree of one small node, depth first, by a warp: a lane per
+// triangle (bounds, bins and the stable partition), then the split as
+// sah_best_split. The triangles and bins live in shared memory; a node of a
+// dozen triangles is some 500 instructions of the warp, where one thread
+// alone took several thousand (0.54 ms for the 10 K subtrees of 200k
+// triangles).
+constexpr int kSmallWarps = 4;
+__global__ void __launch_bounds__(32 * kSmallWarps) k_sah_small(const uint32_t *deferred, uint32_t nd_count,
+                                                               const uint32_t *first_id, SahNodes nd, float4 *plo,
+                                                               float4 *phi, uint32_t *used, uint32_t *max_depth) {
+  struct Work {
+    float4 lo[kSahSmall], hi[kSahSmall];
+    uint32_t bins[kSahBinWords];
+    uint4 task[kSahSmall + 2];  // node, first triangle, count, depth
+  };
+  static_assert(kSahSmall == 32, "a lane per triangle");
+  __shared__ Work work[kSmallWarps];
+  Work &ws = work[threadIdx.x / 32];
+  const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * kSmallWarps, full = 0xffffffffu;
+  for (uint32_t k = blockIdx.x * kSmallWarps + threadIdx.x / 32; k < nd_count; k += warps) {
+    const uint32_t root = deferred[k], base = nd.begin[root], all = nd.count[root], id0 = first_id[k];
+    uint32_t next = id0;
+    if (lane < all) {
+      ws.lo[lane] = plo[base + lane];
+      ws.hi[lane] = phi[base + lane];
+    }
+    int sp = 1;
+    if (lane == 0) ws.task[0] = make_uint4(root, 0, all, nd.depth[root]);
+    __syncwarp();
     while (sp > 0) {
-      const Task t = st[--sp];
-      float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.0f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
-      float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
-      for (uint32_t i = t.b; i < t.b + t.c; ++i) {
-        float l[3], h[3], c[3];
-        prim_box(plo, phi, i, l, h, c);
-        lo = make_float4(fminf(lo.x, l[0]), fminf(lo.y, l[1]), fminf(lo.z, l[2]), 0.0f);
-        hi = make_float4(fmaxf(hi.x, h[0]), fmaxf(hi.y, h[1]), fmaxf(hi.z, h[2]), 0.0f);
-        if (isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2]))
-          for (int q = 0; q < 3; ++q) {
-            clo[q] = fminf(clo[q], c[q]);
-            chi[q] = fmaxf(chi[q], c[q]);
-          }
+      const uint4 t = ws.task[--sp];
+      const uint32_t v = t.x, b0 = t.y, c = t.z, depth = t.w;
+      const bool has = lane < c;
+      float4 l4 = make_float4(INFINITY, INFINITY, INFINITY, 0.0f), h4 = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.0f);
+      if (has) {
+        l4 = ws.lo[b0 + lane];
+        h4 = ws.hi[b0 + lane];
       }
-      nd.lo[t.v] = lo;
-      nd.hi[t.v] = hi;
-      nd.left[t.v] = -1;
-      if (t.c <= 1) {
-        atomicMax(max_depth, t.d);
-        continue;
+      const float l[3] = {l4.x, l4.y, l4.z}, h[3] = {h4.x, h4.y, h4.z};
+      float cen[3];
+      for (int q = 0; q < 3; ++q) cen[q] = (l[q] + h[q]) * 0.5f;
+      const bool ok = has && isfinite(cen[0]) && isfinite(cen[1]) && isfinite(cen[2]);
+      // Bounds as k_sah_bounds: NaN corners are passed over.
+      float nlo[3], nhi[3], clo[3], chi[3], scale[3];
+      bool use[3];
+      for (int q = 0; q < 3; ++q) {
+        nlo[q] = float_of(__reduce_min_sync(full, ord_of(fminf(l[q], INFINITY))));
+        nhi[q] = float_of(__reduce_max_sync(full, ord_of(fmaxf(h[q], -INFINITY))));
+        clo[q] = float_of(__reduce_min_sync(full, ord_of(ok ? cen[q] : INFINITY)));
+        chi[q] = float_of(__reduce_max_sync(full, ord_of(ok ? cen[q] : -INFINITY)));
+        const float span = chi[q] - clo[q];
+        use[q] = span > 0.0f;
+        scale[q] = use[q] ? (float)kSahBins / span : 0.0f;
       }
+      const float4 lo = make_float4(nlo[0], nlo[1], nlo[2], 0.0f), hi = make_float4(nhi[0], nhi[1], nhi[2], 0.0f);
       uint32_t need = 0;
-      for (uint32_t c = t.c; c > kMaxLeafTris; c = (c + 1) / 2) ++need;
-      const bool median = t.d + need >= 56;
-      int axis = -1, best_bin = 0;
-      float best_cost = INFINITY, scale[3] = {0.0f, 0.0f, 0.0f};
-      if (!median) {
-        const float parent = host_area(lo, hi);
-        for (int ax = 0; ax < 3; ++ax) {
-          const float span = chi[ax] - clo[ax];
-          if (!(span > 0.0f)) continue;
-          scale[ax] = (float)kSahBins / span;
-          uint32_t bc[kSahBins];
-          float bl[kSahBins][3], bh[kSahBins][3];
-          for (int b = 0; b < kSahBins; ++b) {
-            bc[b] = 0;
-            for (int q = 0; q < 3; ++q) {
-              bl[b][q] = INFINITY;
-              bh[b][q] = -INFINITY;
-            }
-          }
-          for (uint32_t i = t.b; i < t.b + t.c; ++i) {
-            float l[3], h[3], c[3];
-            prim_box(plo, phi, i, l, h, c);
-            const int b = sah_bin((c[ax] - clo[ax]) * scale[ax]);
-            bc[b]++;
-            for (int q = 0; q < 3; ++q) {
-              bl[b][q] = fminf(bl[b][q], l[q]);
-              bh[b][q] = fmaxf(bh[b][q], h[q]);
-            }
-          }
-          float rl[kSahBins][3], rh[kSahBins][3];
-          uint32_t rc[kSahBins];
-          float accl[3] = {INFINITY, INFINITY, INFINITY}, acch[3] = {-INFINITY, -INFINITY, -INFINITY};
-          uint32_t acc = 0;
-          for (int b = kSahBins - 1; b >= 1; --b) {
-            acc += bc[b];
-            for (int q = 0; q < 3; ++q) {
-              accl[q] = fminf(accl[q], bl[b][q]);
-              acch[q] = fmaxf(acch[q], bh[b][q]);
-              rl[b][q] = accl[q];
-              rh[b][q] = acch[q];
-            }
-            rc[b] = acc;
-          }
-          float ll[3] = {INFINITY, INFINITY, INFINITY}, lh[3] = {-INFINITY, -INFINITY, -INFINITY};
-          uint32_t lc = 0;
-          for (int s = 1; s < kSahBins; ++s) {
-            lc += bc[s - 1];
-            for (int q = 0; q < 3; ++q) {
-              ll[q] = fminf(ll[q], bl[s - 1][q]);
-              lh[q] = fmaxf(lh[q], bh[s - 1][q]);
-            }
-            if (lc == 0 || rc[s] == 0) continue;
-            const float cost = 1.0f + (host_area(make_float4(ll[0], ll[1], ll[2], 0.0f), make_float4(lh[0], lh[1], lh[2], 0.0f)) *
-                                           (float)lc +
-                                       host_area(make_float4(rl[s][0], rl[s][1], rl[s][2], 0.0f),
-                                                 make_float4(rh[s][0], rh[s][1], rh[s][2], 0.0f)) *
-                                           (float)rc[s]) /
-                                          fmaxf(parent, 1e-30f);
-            if (cost < best_cost) {
-              best_cost = cost;
-              axis = ax;
-              best_bin = s;
-            }
-          }
+      for (uint32_t x = c; x > kMaxLeafTris; x = (x + 1) / 2) ++need;
+      uint32_t split = kSahHalve;
+      if (c <= 1) {
+        split = kSahNone;
+      } else if (depth + need < 56) {
+        for (int w = lane; w < kSahBinWords; w += 32) {
+          const int f = w % 7;
+          ws.bins[w] = (f >= 1 && f <= 3) ? 0xffffffffu : 0u;
         }
-        if (t.c <= kMaxLeafTris && (axis < 0 || (float)t.c <= best_cost)) {
-          atomicMax(max_depth, t.d);
-          continue;
-        }
+        __syncwarp();
+        if (has) sah_add_bins<true>(ws.bins, l, h, cen, clo, scale, use);
+        __syncwarp();
+        float cost;
+        const uint32_t at = sah_best_split(ws.bins, use, host_area(lo, hi), cost);
+        if (at != kSahNone) split = at;
+        if (c <= kMaxLeafTris && (at == kSahNone || (float)c <= cost)) split = kSahNone;
       }
-      uint32_t mid;
-      if (axis >= 0) {
-        uint32_t i = t.b, j = t.b + t.c;  // [t.b, i) left, [j, end) right
-        while (i < j) {
-          float l[3], h[3], c[3];
-          prim_box(plo, phi, i, l, h, c);
-          if (sah_bin((c[axis] - clo[axis]) * scale[axis]) < best_bin) {
-            ++i;
-          } else {
-            --j;
-            const float4 a = plo[i], b = phi[i];
-            plo[i] = plo[j];
-            phi[i] = phi[j];
-            plo[j] = a;
-            phi[j] = b;
-          }
+      if (lane == 0) {
+        nd.lo[v] = lo;
+        nd.hi[v] = hi;
+        nd.left[v] = split == kSahNone ? -1 : (int)next;
+        if (split == kSahNone) atomicMax(max_depth, depth);
+      }
+      if (split == kSahNone) continue;
+      uint32_t mid = c / 2;
+      if (split != kSahHalve) {
+        const uint32_t axis = split >> 8;
+        const float f = axis == 0 ? (cen[0] - clo[0]) * scale[0]
+                                  : (axis == 1 ? (cen[1] - clo[1]) * scale[1] : (cen[2] - clo[2]) * scale[2]);
+        const bool left = has && sah_bin(f) < (int)(split & 0xffu);
+        const uint32_t lm = __ballot_sync(full, left), before = (1u << lane) - 1u;
+        mid = __popc(lm);
+        __syncwarp();
+        if (has) {
+          const uint32_t to = b0 + (left ? __popc(lm & before) : mid + lane - __popc(lm & before));
+          ws.lo[to] = l4;
+          ws.hi[to] = h4;
         }
-        mid = i - t.b;
-      } else {
-        mid = t.c / 2;
       }
       const uint32_t c0 = next;
       next += 2;
-      nd.left[t.v] = (int)c0;
-      nd.begin[c0] = t.b;
-      nd.count[c0] = mid;
-      nd.begin[c0 + 1] = t.b + mid;
-      nd.count[c0 + 1] = t.c - mid;
-      nd.depth[c0] = nd.depth[c0 + 1] = t.d + 1;
-      st[sp++] = {c0 + 1, t.b + mid, t.c - mid, t.d + 1};
-      st[sp++] = {c0, t.b, mid, t.d + 1};
+      if (lane == 0) {
+        nd.begin[c0] = base + b0;
+        nd.count[c0] = mid;
+        nd.begin[c0 + 1] = base + b0 + mid;
+        nd.count[c0 + 1] = c - mid;
+        nd.depth[c0] = nd.depth[c0 + 1] = depth + 1;
+        ws.task[sp] = make_uint4(c0 + 1, b0 + mid, c - mid, depth + 1);
+        ws.task[sp + 1] = make_uint4(c0, b0, mid, depth + 1);
+      }
+      sp += 2;
+      __syncwarp();
     }
-    used[k] = next - id0;
+    __syncwarp();
+    if (lane < all) {
+      plo[base + lane] = ws.lo[lane];
+      phi[base + lane] = ws.hi[lane];
+    }
+    if (lane == 0) used[k] = next - id0;
+    __syncwarp();
   }
 }
 
@@ -1293,12 +1321,13 @@ __global__ void k_sah_root(SahNodes nd, uint32_t n, uint32_t *act) {
 struct Scratch {
   std::vector<void *> ptrs;
   cudaStream_t st;
+  cudaMemPool_t pool;
   bool oom = false;
   std::string err;
   template <class T>
   T *get(uint64_t count) {
     void *p = nullptr;
-    cudaError_t e = cudaMallocAsync(&p, std::max<uint64_t>(count, 1) * sizeof(T), st);
+    cudaError_t e = device_alloc(&p, std::max<uint64_t>(count, 1) * sizeof(T), st, pool);
     if (e != cudaSuccess) {
       cudaGetLastError();
       if (err.empty()) err = std::string("device BVH scratch allocation failed: ") + cudaGetErrorString(e);
@@ -1318,7 +1347,7 @@ uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 }  // namespace
 
 std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t st, uint32_t max_depth_allowed, bool &oom,
-                                 DeviceBuildInfo *info) {
+                                 DeviceBuildInfo *info, cudaMemPool_t pool) {
   oom = false;
   const auto t0 = std::chrono::steady_clock::now();
   const uint64_t n64 = sc.tri_count;
@@ -1327,7 +1356,7 @@ std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t st, uint32_t max_de
   const uint32_t n = (uint32_t)n64;
   const uint32_t cap = 2 * n;  // nodes of a binary tree with non-empty leaves
 
-  Scratch s{{}, st};
+  Scratch s{{}, st, pool};
   float4 *plo = s.get<float4>(n), *phi = s.get<float4>(n), *qlo = s.get<float4>(n), *qhi = s.get<float4>(n);
   uint32_t *seg = s.get<uint32_t>(n), *flag = s.get<uint32_t>(n), *pscan = s.get<uint32_t>(n);
   uint32_t *scan32 = s.get<uint32_t>(scan_scratch_items(n));
@@ -1379,9 +1408,9 @@ std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t st, uint32_t max_de
     k_sah_init_bins<<<grid_for((uint64_t)m * kSahBinWords), kThreads, 0, st>>>(lv);
     k_sah_seg<<<grid_for(n), kThreads, 0, st>>>(nd, lv, n, seg);
     k_sah_bounds<<<grid_for(n), kThreads, 0, st>>>(plo, phi, seg, n, lv);
-    k_sah_bins<<<(unsigned)std::min<uint64_t>(tiles_of(n, kThreads * 8), 1u << 16), kThreads, 0, st>>>(plo, phi, seg,
+    k_sah_bins<<<(unsigned)std::min<uint64_t>(tiles_of(n, kSahBinTile), 1u << 16), kThreads, 0, st>>>(plo, phi, seg,
                                                                                                   n, lv);
-    k_sah_split<<<grid_for(m), kThreads, 0, st>>>(nd, lv, counters);
+    k_sah_split<<<grid_for(32ull * m), kThreads, 0, st>>>(nd, lv, counters);
     k_sah_flags<<<grid_for(n), kThreads, 0, st>>>(plo, phi, seg, n, lv, flag);
     scan_exclusive<uint32_t>(flag, pscan, n, scan32, st);
     k_sah_scatter<<<grid_for(n), kThreads, 0, st>>>(plo, phi, qlo, qhi, seg, flag, pscan, n, nd, lv);
@@ -1423,7 +1452,7 @@ std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t st, uint32_t max_de
     if ((uint64_t)next_id + reserved > cap) return "device SAH build ran out of nodes";
     if (reserved) k_sah_small_clear<<<grid_for(reserved), kThreads, 0, st>>>(nd, next_id, next_id + reserved);
     k_add_base<<<grid_for(n_deferred), kThreads, 0, st>>>(first_id, n_deferred, next_id);
-    k_sah_small<<<grid_for(n_deferred, 64), 64, 0, st>>>(deferred, n_deferred, first_id, nd, plo, phi, used, counters);
+    k_sah_small<<<grid_for(n_deferred, kSmallWarps), 32 * kSmallWarps, 0, st>>>(deferred, n_deferred, first_id, nd, plo, phi, used, counters);
     next_id += reserved;
   }
   const uint32_t total = next_id;
@@ -1453,13 +1482,14 @@ std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t st, uint32_t max_de
   const uint64_t offr = off4 + align256((uint64_t)n4 * sizeof(Bvh4Node));
   const uint64_t bytes = offr + align256(3ull * n * sizeof(float4));
   DeviceArena arena;
-  e = cudaMalloc(&arena.base, bytes);
+  e = device_alloc(&arena.base, bytes, pool ? st : nullptr, pool);
   if (e != cudaSuccess) {
     cudaGetLastError();
     oom = e == cudaErrorMemoryAllocation;
     return std::string("device allocation of ") + std::to_string(bytes) + " BVH bytes failed: " + cudaGetErrorString(e);
   }
   arena.bytes = bytes;
+  arena.stream = pool ? st : nullptr;
   uint8_t *base = static_cast<uint8_t *>(arena.base);
   BvhNode *out2 = reinterpret_cast<BvhNode *>(base);
   Bvh4Node *out4 = reinterpret_cast<Bvh4Node *>(base + off4);
@@ -1498,7 +1528,7 @@ std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t st, uint32_t max_de
 }
 
 std::string device_build_bvh(SceneHost &sc, cudaStream_t st, uint32_t max_depth_allowed, bool &oom,
-                             DeviceBuildInfo *info) {
+                             DeviceBuildInfo *info, cudaMemPool_t pool) {
   oom = false;
   const auto t0 = std::chrono::steady_clock::now();
   const uint64_t n64 = sc.tri_count;
@@ -1507,7 +1537,7 @@ std::string device_build_bvh(SceneHost &sc, cudaStream_t st, uint32_t max_depth_
   const uint32_t n = (uint32_t)n64;
   const uint32_t total_nodes = 2 * n - 1;
 
-  Scratch s{{}, st};
+  Scratch s{{}, st, pool};
   float4 *plo = s.get<float4>(n), *phi = s.get<float4>(n);
   uint32_t *cb = s.get<uint32_t>(6);
   MortonKey *keys = s.get<MortonKey>(n), *keys2 = s.get<MortonKey>(n);
@@ -1614,13 +1644,14 @@ std::string device_build_bvh(SceneHost &sc, cudaStream_t st, uint32_t max_depth_
   const uint64_t offr = off4 + align256((uint64_t)n4 * sizeof(Bvh4Node));
   const uint64_t bytes = offr + align256(3ull * n * sizeof(float4));
   DeviceArena arena;
-  e = cudaMalloc(&arena.base, bytes);
+  e = device_alloc(&arena.base, bytes, pool ? st : nullptr, pool);
   if (e != cudaSuccess) {
     cudaGetLastError();
     oom = e == cudaErrorMemoryAllocation;
     return std::string("device allocation of ") + std::to_string(bytes) + " BVH bytes failed: " + cudaGetErrorString(e);
   }
   arena.bytes = bytes;
+  arena.stream = pool ? st : nullptr;
   uint8_t *base = static_cast<uint8_t *>(arena.base);
   BvhNode *out2 = reinterpret_cast<BvhNode *>(base);
   Bvh4Node *out4 = reinterpret_cast<Bvh4Node *>(base + off4);

@@ -39,7 +39,7 @@ struct DeviceBuildInfo {
 // starts with "depth" and leaves `sc` unchanged; the caller then builds on
 // the host. `oom` is set when the failure was a device allocation.
 std::string device_build_bvh(SceneHost &sc, cudaStream_t stream, uint32_t max_depth, bool &oom,
-                             DeviceBuildInfo *info = nullptr);
+                             DeviceBuildInfo *info = nullptr, cudaMemPool_t pool = nullptr);
 
 // The same contract with the host builder's binned-SAH split rule, built
 // top down one tree level per round: per active node its bounds, 16 bins
@@ -48,6 +48,6 @@ std::string device_build_bvh(SceneHost &sc, cudaStream_t stream, uint32_t max_de
 // at the depth limit or without a valid split halve their range by index
 // (the host splits at the centroid median there).
 std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t stream, uint32_t max_depth, bool &oom,
-                                 DeviceBuildInfo *info = nullptr);
+                                 DeviceBuildInfo *info = nullptr, cudaMemPool_t pool = nullptr);
 
 }  // namespace ptd

@@ -231,7 +231,7 @@ uint32_t grid_of(uint64_t n) {
 
 }  // namespace
 
-std::string device_refit_bvh(SceneHost &sc, uint64_t records, cudaStream_t st) {
+std::string device_refit_bvh(SceneHost &sc, uint64_t records, cudaStream_t st, cudaMemPool_t pool) {
   DevScene &d = sc.dev;
   if (!d.nodes && !d.nodes4) return "";
   float4 *rec = const_cast<float4 *>(d.tris);
@@ -242,7 +242,7 @@ std::string device_refit_bvh(SceneHost &sc, uint64_t records, cudaStream_t st) {
   uint32_t *scratch = nullptr;
   // Links and counts of either layout, then the four-child nodes' bounds.
   const uint64_t links = (2 * nmax * sizeof(uint32_t) + 255) & ~uint64_t(255);
-  cudaError_t e = cudaMallocAsync((void **)&scratch, links + 2 * (uint64_t)n4 * sizeof(float4), st);
+  cudaError_t e = device_alloc((void **)&scratch, links + 2 * (uint64_t)n4 * sizeof(float4), st, pool);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return std::string("refit scratch: ") + cudaGetErrorString(e);

@@ -836,6 +836,17 @@ pt_status engine_create(int device, pt_context **out) {
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
+  int pools = 0;
+  if (e == cudaSuccess && cudaDeviceGetAttribute(&pools, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && pools) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    uint64_t keep = pt_context::kPoolKeep;
+    if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess) ctx->pool = nullptr;
+    if (ctx->pool) cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    cudaGetLastError();
+  }
   if (e != cudaSuccess) {
     pt_destroy(ctx.release());
     return fail(nullptr, PT_ERR_DEVICE, std::string("context setup failed: ") + cudaGetErrorString(e));
@@ -881,6 +892,8 @@ void pt_destroy(pt_context *ctx) {
   for (cudaEvent_t ev : ctx->stage_events) cudaEventDestroy(ev);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+  if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   ctx->staging.release();
   delete ctx;
@@ -896,7 +909,7 @@ pt_status pt_scene_upload(pt_context *ctx, const pt_scene_desc *desc, uint32_t *
     auto sc = std::make_unique<SceneHost>();
     if (injected_oom(ctx)) return fail(ctx, PT_ERR_OOM, "scene upload: device allocation failed (injected)");
     bool oom = false;
-    std::string err = upload_scene(*desc, *sc, oom, ctx->bvh_builder, ctx->stream, &ctx->staging);
+    std::string err = upload_scene(*desc, *sc, oom, ctx->bvh_builder, ctx->stream, &ctx->staging, ctx->pool);
     if (!err.empty()) return fail(ctx, oom ? PT_ERR_OOM : PT_ERR_INVALID_ARG, err);
     uint32_t id = ctx->next_id++;
     ctx->scenes[id] = std::move(sc);
@@ -929,7 +942,7 @@ pt_status pt_scene_refit(pt_context *ctx, uint32_t scene_id, const pt_scene_desc
     CK(ctx, cudaStreamSynchronize(ctx->stream));
     if (injected_oom(ctx)) return fail(ctx, PT_ERR_OOM, "scene refit: device allocation failed (injected)");
     bool oom = false;
-    std::string err = refit_scene(*desc, *sc, oom, ctx->stream, &ctx->staging);
+    std::string err = refit_scene(*desc, *sc, oom, ctx->stream, &ctx->staging, ctx->pool);
     if (!err.empty()) return fail(ctx, oom ? PT_ERR_OOM : PT_ERR_INVALID_ARG, err);
     return PT_OK;
   });
@@ -1252,7 +1265,7 @@ pt_status pt_raycast_render(pt_context *ctx, uint32_t scene_id, const pt_camera 
     const uint64_t off_deep = off_ovf + (pbr ? al(ns * sizeof(uint32_t)) : 0);
     const uint64_t total = off_deep + (pbr ? al((uint64_t)deep_slots * raycast_pbr_frame_bytes()) : 0);
     void *buf = nullptr;
-    CK(ctx, cudaMallocAsync(&buf, total, ctx->stream));
+    CK(ctx, device_alloc(&buf, total, ctx->stream, ctx->pool));
     std::unique_ptr<void, std::function<void(void *)>> hold(buf, [ctx](void *q) { cudaFreeAsync(q, ctx->stream); });
     uint8_t *b = static_cast<uint8_t *>(buf);
     uint32_t *d_err = reinterpret_cast<uint32_t *>(b + off_err);

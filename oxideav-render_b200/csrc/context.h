@@ -50,6 +50,13 @@ struct pt_context {
   uint32_t trav_threads = 256;  // traversal kernels' block size (128 or 256; 1,024 threads per SM)
   uint32_t claim_chunk = 1;     // queue entries a traversal lane claims per refill (1, 2 or 4)
   int bvh_builder = ptd::BVH_BUILD_AUTO;  // where pt_scene_upload builds the BVH (ptd::BvhBuilder)
+  // Device memory of scenes, trees, build scratch and raycast frames: a
+  // one-shot render takes and returns some 70 MB, which the pool keeps (up to
+  // kPoolKeep; returned with the context) instead of unmapping at every
+  // release. Every allocation is made, used and freed on `stream`, or between
+  // synchronisations with it. nullptr where the device has no pools.
+  cudaMemPool_t pool = nullptr;
+  static constexpr uint64_t kPoolKeep = 1ull << 30;
   ptd::HostStaging staging;  // pinned host image buffer of pt_scene_upload
   std::map<uint32_t, ptd::TuneChoice> tuned;  // by scene class (ptd::scene_class)
   // Wavefront waves replayed as CUDA graphs (bounce count << 1 | sort -> exec).

@@ -1124,6 +1124,16 @@ void emit_tree(const std::vector<BNode> &in_nodes, const std::vector<uint32_t> &
 }  // namespace
 
 // ============================================================ arena
+cudaError_t device_alloc(void **p, uint64_t bytes, cudaStream_t stream, cudaMemPool_t pool) {
+  if (!pool) return stream ? cudaMallocAsync(p, bytes, stream) : cudaMalloc(p, bytes);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  cudaStreamSynchronize(stream);
+  cudaMemPoolTrimTo(pool, 0);
+  return cudaMallocFromPoolAsync(p, bytes, pool, stream);
+}
+
 void DeviceArena::release() {
   if (base) {
     if (stream)
@@ -1618,12 +1628,12 @@ void rebase(const P *&p, uint8_t *base) {
 // Allocates `a` for `t` and copies it (stream-ordered when `stream` is
 // non-null), pointing d's tree fields into it.
 std::string commit_tree(const HostTree &t, uint32_t max_depth, DeviceArena &a, DevScene &d, bool &oom,
-                        cudaStream_t stream) {
+                        cudaStream_t stream, cudaMemPool_t pool) {
   auto al = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
   const uint64_t b2 = t.nodes.size() * sizeof(BvhNode), b4 = t.nodes4.size() * sizeof(Bvh4Node);
   const uint64_t br = t.records.size() * sizeof(float4);
   const uint64_t off4 = al(b2), offr = off4 + al(b4), total = std::max<uint64_t>(offr + al(br), 256);
-  cudaError_t e = stream ? cudaMallocAsync(&a.base, total, stream) : cudaMalloc(&a.base, total);
+  cudaError_t e = device_alloc(&a.base, total, stream, pool);
   if (e != cudaSuccess) {
     oom = e == cudaErrorMemoryAllocation;
     a.base = nullptr;
@@ -1654,10 +1664,10 @@ std::string commit_tree(const HostTree &t, uint32_t max_depth, DeviceArena &a, D
 
 }  // namespace
 
-std::string commit_scene(const SceneImage &img, SceneHost &out, bool &oom, cudaStream_t stream) {
+std::string commit_scene(const SceneImage &img, SceneHost &out, bool &oom, cudaStream_t stream, cudaMemPool_t pool) {
   oom = false;
   const size_t total = std::max<uint64_t>(img.blob.size(), img.pool_off + img.pool_bytes);
-  cudaError_t e = stream ? cudaMallocAsync(&out.arena.base, total, stream) : cudaMalloc(&out.arena.base, total);
+  cudaError_t e = device_alloc(&out.arena.base, total, stream, pool);
   if (e != cudaSuccess) {
     oom = e == cudaErrorMemoryAllocation;
     out.arena.base = nullptr;
@@ -1710,7 +1720,7 @@ std::string commit_scene(const SceneImage &img, SceneHost &out, bool &oom, cudaS
     }
   }
   if (!img.tree.nodes.empty()) {
-    std::string err = commit_tree(img.tree, img.bvh.max_depth, out.bvh_arena, d, oom, stream);
+    std::string err = commit_tree(img.tree, img.bvh.max_depth, out.bvh_arena, d, oom, stream, pool);
     if (!err.empty()) {
       out.arena.release();
       return err;
@@ -1732,8 +1742,23 @@ std::string commit_scene(const SceneImage &img, SceneHost &out, bool &oom, cudaS
 }
 
 std::string upload_scene(const pt_scene_desc &desc, SceneHost &out, bool &oom, int builder, cudaStream_t stream,
-                         HostStaging *staging) {
+                         HostStaging *staging, cudaMemPool_t pool) {
   oom = false;
+  // Commits on the stream from the pool where there is one. Whatever is
+  // staged is copied, and the scene whole, when this returns.
+  cudaStream_t cs = pool ? stream : nullptr;
+  auto commit = [&](const SceneImage &img) {
+    std::string err = commit_scene(img, out, oom, cs, pool);
+    if (err.empty() && cs) {
+      const cudaError_t e = cudaStreamSynchronize(cs);
+      if (e != cudaSuccess) {
+        err = std::string("scene upload failed: ") + cudaGetErrorString(e);
+        out.arena.release();
+        out.bvh_arena.release();
+      }
+    }
+    return err;
+  };
   out.item_tris.clear();
   for (uint32_t i = 0; desc.items && i < desc.item_count; ++i) out.item_tris.push_back(desc.items[i].triangle_count);
   using clk = std::chrono::steady_clock;
@@ -1748,11 +1773,11 @@ std::string upload_scene(const pt_scene_desc &desc, SceneHost &out, bool &oom, i
     std::string err = build_scene_image(desc, img, false, staging);
     if (!err.empty()) return err;
     const auto t1 = clk::now();
-    err = commit_scene(img, out, oom);
+    err = commit(img);
     if (!err.empty()) return err;
     const auto t2 = clk::now();
-    err = builder == BVH_BUILD_DEVICE_PLOC ? device_build_bvh(out, stream, kMaxTreeDepth, oom)
-                                           : device_build_bvh_sah(out, stream, kMaxTreeDepth, oom);
+    err = builder == BVH_BUILD_DEVICE_PLOC ? device_build_bvh(out, stream, kMaxTreeDepth, oom, nullptr, pool)
+                                           : device_build_bvh_sah(out, stream, kMaxTreeDepth, oom, nullptr, pool);
     if (err.empty()) {
       const auto t3 = clk::now();
       out.upload_seconds[0] = secs(t0, t1);
@@ -1771,7 +1796,7 @@ std::string upload_scene(const pt_scene_desc &desc, SceneHost &out, bool &oom, i
   std::string err = build_scene_image(desc, img, true, nullptr, builder == BVH_BUILD_HOST_SPATIAL);
   if (!err.empty()) return err;
   const auto t2 = clk::now();
-  err = commit_scene(img, out, oom);
+  err = commit(img);
   const auto t3 = clk::now();
   out.upload_seconds[0] = secs(t1, t2);
   out.upload_seconds[1] = secs(t2, t3);
@@ -1781,7 +1806,7 @@ std::string upload_scene(const pt_scene_desc &desc, SceneHost &out, bool &oom, i
 }
 
 std::string refit_scene(const pt_scene_desc &desc, SceneHost &sc, bool &oom, cudaStream_t stream,
-                        HostStaging *staging) {
+                        HostStaging *staging, cudaMemPool_t pool) {
   oom = false;
   using clk = std::chrono::steady_clock;
   auto secs = [](clk::time_point a, clk::time_point b) { return std::chrono::duration<double>(b - a).count(); };
@@ -1795,7 +1820,7 @@ std::string refit_scene(const pt_scene_desc &desc, SceneHost &sc, bool &oom, cud
   if (!err.empty()) return err;
   const auto t1 = clk::now();
   SceneHost fresh;
-  err = commit_scene(img, fresh, oom, stream);
+  err = commit_scene(img, fresh, oom, stream, pool);
   if (!err.empty()) return err;
   const auto t2 = clk::now();
   // The old tree, refitted to the new positions, goes with the new arena.
@@ -1809,7 +1834,7 @@ std::string refit_scene(const pt_scene_desc &desc, SceneHost &sc, bool &oom, cud
   fresh.bvh = sc.bvh;
   fresh.device_bvh = sc.device_bvh;
   fresh.item_tris = sc.item_tris;
-  err = device_refit_bvh(fresh, sc.bvh.references, stream);
+  err = device_refit_bvh(fresh, sc.bvh.references, stream, pool);
   cudaError_t e = cudaSuccess;
   if (err.empty()) e = cudaMemcpyAsync(fresh.d_desc, &fresh.dev, sizeof(DevScene), cudaMemcpyHostToDevice, stream);
   if (err.empty() && e == cudaSuccess) e = cudaStreamSynchronize(stream);

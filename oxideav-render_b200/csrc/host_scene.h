@@ -38,6 +38,12 @@ void build_bvh_spatial(const float *pos, uint32_t tri_count, const uint32_t *rec
 // One device allocation holding a scene (or an environment) plus the
 // device copy of its descriptor. `stream` non-null: the allocation is
 // stream-ordered (cudaMallocAsync) and is freed in that stream's order.
+// Device memory for scenes, their trees and build scratch: from `pool`
+// (stream-ordered; the context's, see pt_context::pool), else from the
+// device's default pool on `stream`, else synchronously. A pool that cannot
+// serve the request gives its cached memory back first and is asked again.
+cudaError_t device_alloc(void **p, uint64_t bytes, cudaStream_t stream, cudaMemPool_t pool);
+
 struct DeviceArena {
   void *base = nullptr;
   uint64_t bytes = 0;
@@ -139,7 +145,8 @@ std::string build_scene_image(const pt_scene_desc &desc, SceneImage &img, bool w
                               HostStaging *staging = nullptr, bool spatial = false);
 // Allocates the arena and copies `img` into it (stream-ordered when `stream`
 // is non-null). `oom` is set when the failure was a device allocation.
-std::string commit_scene(const SceneImage &img, SceneHost &out, bool &oom, cudaStream_t stream = nullptr);
+std::string commit_scene(const SceneImage &img, SceneHost &out, bool &oom, cudaStream_t stream = nullptr,
+                         cudaMemPool_t pool = nullptr);
 // Deepest leaf a tree may have: the traversal stacks hold 64 two-child
 // entries and 3 * 56 + 8 four-child entries.
 constexpr uint32_t kMaxTreeDepth = 56;
@@ -162,7 +169,8 @@ constexpr uint64_t kAutoDeviceBuildTris = 16384;
 // says (`stream`: the device build's stream). A device-built tree deeper
 // than the traversal stacks allow is rebuilt on the host.
 std::string upload_scene(const pt_scene_desc &desc, SceneHost &out, bool &oom, int builder = BVH_BUILD_HOST,
-                         cudaStream_t stream = nullptr, HostStaging *staging = nullptr);
+                         cudaStream_t stream = nullptr, HostStaging *staging = nullptr,
+                         cudaMemPool_t pool = nullptr);
 void release_scene(SceneHost &s);
 // An animated frame of a resident scene with the same draw items and
 // triangle counts: the new host image (no BVH) replaces the scene arena, the
@@ -170,10 +178,10 @@ void release_scene(SceneHost &s);
 // (device_refit_bvh). upload_seconds then holds: host image, arena copy,
 // refit, total.
 std::string refit_scene(const pt_scene_desc &desc, SceneHost &sc, bool &oom, cudaStream_t stream,
-                        HostStaging *staging);
+                        HostStaging *staging, cudaMemPool_t pool = nullptr);
 // Records rewritten from the scene's positions and both node layouts'
 // bounds recomputed bottom up (bvh_refit.cu); `records` triangle records.
-std::string device_refit_bvh(SceneHost &sc, uint64_t records, cudaStream_t stream);
+std::string device_refit_bvh(SceneHost &sc, uint64_t records, cudaStream_t stream, cudaMemPool_t pool = nullptr);
 struct EnvHost {
   DevEnv dev{};
   DevEnv *d_desc = nullptr;

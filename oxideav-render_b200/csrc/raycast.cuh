@@ -22,6 +22,10 @@ constexpr float kLegacyAmbient = 0.2f;          // AMBIENT, src/shade.rs:13
 constexpr float kSecondaryRayThreshold = 1.0e-2f;  // src/raycast.rs:130
 constexpr float kWireframeEdge = 0.03f;          // src/raycast.rs:134
 
+// Rays walk the two-child layout: a frame's recursion stack and the wider
+// visit's registers together cost more than its fewer steps save (sphere
+// grid 512x512, aa 2: 1.28 ms, with the four-child layout 1.47). Pbr mode,
+// whose rays also feed any-hit filters, gains from it: 1.00 -> 0.91 ms.
 struct RaycastParams {
   DevScene s;
   pt_camera cam;
@@ -137,7 +141,7 @@ PT_DEV bool whitted_enter(const RaycastParams &p, WhittedFrame &f, V3 d, const H
   f.skip = h.g;
   V3 so = offset_ray_origin(f.p, f.n);
   TraversalStats st{0, 0};
-  bool shadowed = occluded(s, so, p.light_dir, 0.0f, inf(), AcceptNotSelf{f.skip}, st, err);
+  bool shadowed = occluded<false>(s, so, p.light_dir, 0.0f, inf(), AcceptNotSelf{f.skip}, st, err);
   f.out = shadowed ? make_float4(f.a.x * kLegacyAmbient, f.a.y * kLegacyAmbient, f.a.z * kLegacyAmbient, f.a.w)
                    : shade_legacy(f.a, f.n, p.light_dir, p.light_intensity);
   f.out.x += m.emissive[0];
@@ -216,7 +220,7 @@ PT_DEV float4 whitted(const RaycastParams &p, V3 d0, const Hit &h0, uint32_t &er
     if (!child) continue;
     Hit h;
     TraversalStats st{0, 0};
-    if (!closest_hit(p.s, o, dir, 0.0f, inf(), AcceptNotSelf{f.skip}, h, st, err)) {
+    if (!closest_hit<false>(p.s, o, dir, 0.0f, inf(), AcceptNotSelf{f.skip}, h, st, err)) {
       // Escaping rays: black for the mirror ray, nothing through the
       // transmission, no change for total internal reflection.
       if (how == 1) whitted_combine(f, 1, make_float4(0.0f, 0.0f, 0.0f, 1.0f));
@@ -255,7 +259,7 @@ __global__ void __launch_bounds__(128) k_raycast(RaycastParams p) {
     }
     Hit h;
     TraversalStats st{0, 0};
-    bool covered = closest_hit(p.s, o, d, 0.0f, inf(), AcceptAll{}, h, st, err);
+    bool covered = closest_hit<false>(p.s, o, d, 0.0f, inf(), AcceptAll{}, h, st, err);
     float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (covered) {
       const pt_material &m = p.s.materials[__ldg(p.s.tri_info + h.g).x].m;

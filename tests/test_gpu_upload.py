@@ -1,0 +1,112 @@
+"""Scene uploads: the device binned-SAH build at the sizes where its kernels
+change hands (64 triangles is its least, subtrees of at most 32 go to a warp,
+tiles of 1,024), with coinciding, flat and NaN triangles, against the host
+build; and the context's memory pool over many uploads and two threads."""
+import threading
+
+import numpy as np
+import pytest
+
+from oxideav_render_b200 import abi, api, testscenes as ts
+from oxideav_render_b200.scene import PreparedScene, Primitive
+
+pytestmark = pytest.mark.gpu
+
+
+def cloud(kind, n, seed=1):
+    rng = np.random.default_rng(seed + n)
+    c = rng.random((n, 1, 3)).astype(np.float32)
+    e = (rng.normal(size=(n, 3, 3)) * 0.03).astype(np.float32)
+    pos = c + e
+    if kind == "same":  # every centroid alike: no split plane, ranges are halved
+        pos[:] = pos[0]
+    elif kind == "flat":
+        pos[..., 1] = 0.5
+    elif kind == "piles":  # a few places, many triangles each
+        pos = (np.round(c * 2) / 2 + e * 0.01).astype(np.float32)
+    elif kind == "nan":
+        pos[::7, 1, 2] = np.nan
+    s = PreparedScene()
+    m = s.add_material(ts.diffuse_material((0.7, 0.6, 0.5), 1.0))
+    s.add_primitive(Primitive(np.ascontiguousarray(pos.reshape(-1, 3).astype(np.float32)), material=m))
+    s.add_camera([0.5, 0.6, 2.4], [0.5, 0.5, 0.5], 0.6)
+    return s
+
+
+def render(ctx, scene, opts):
+    t = api.PathTracer(ctx)
+    t.sync(scene, opts)
+    t.refine(opts.path_trace.samples_per_pixel)
+    out = t.accum(), ctx.bvh_stats(t.scene_id), ctx.bvh_on_device(t.scene_id)
+    t.close()
+    return out
+
+
+@pytest.mark.parametrize("n", [64, 65, 97, 1023, 1025, 4097])
+@pytest.mark.parametrize("kind", ["random", "same", "flat", "piles", "nan"])
+def test_device_build_equals_the_host_build(ctx, kind, n):
+    scene, o = cloud(kind, n), ts.pt_opts(33, 2, 4, h=31, ambient=0.5)
+    out = {}
+    for b in (abi.PT_BVH_BUILD_HOST, abi.PT_BVH_BUILD_DEVICE):
+        ctx.set_bvh_builder(b)
+        try:
+            out[b] = render(ctx, scene, o)
+        finally:
+            ctx.set_bvh_builder(abi.PT_BVH_BUILD_AUTO)
+    (a, sa, _), (b, sb, on_device) = out[abi.PT_BVH_BUILD_HOST], out[abi.PT_BVH_BUILD_DEVICE]
+    # NaN triangles leave the scene; what is left may be too few for the device.
+    assert (on_device or (kind == "nan" and n < 97)) and np.array_equal(a, b)
+    if kind in ("random", "flat"):  # no fallback splits: the same tree
+        assert (sa["nodes"], sa["leaves"], sa["max_depth"]) == (sb["nodes"], sb["leaves"], sb["max_depth"])
+        assert sa["sah_cost"] == pytest.approx(sb["sah_cost"], rel=1e-9)
+
+
+def test_pool_keeps_a_bounded_cache():
+    import torch
+    scene, o = cloud("random", 50000), ts.pt_opts(16, 1, 2, ambient=0.5)
+    c = api.Context(0)
+    try:
+        d = scene.to_desc(o)
+        want = None
+        ids = []
+        for k in range(40):
+            ids.append(c.upload(d))
+            if k % 3:
+                c.release(ids.pop(0))
+            if k % 10 == 5:
+                got = render(c, scene, o)[0]
+                want = got if want is None else want
+                assert np.array_equal(got, want)
+        held = torch.cuda.mem_get_info()[0]
+        for i in ids:
+            c.release(i)
+        # Released scenes stay in the pool up to its limit, no further.
+        big = ts.stress_c2(64, 64, 1, grid=512, spheres=50)[0].to_desc(o)
+        for _ in range(3):
+            c.release(c.upload(big))
+        assert held - torch.cuda.mem_get_info()[0] < 3 << 29
+    finally:
+        c.close()
+
+
+def test_two_contexts_in_two_threads():
+    scenes = [cloud("random", 20000, 1), cloud("piles", 30000, 2)]
+    o = ts.pt_opts(40, 2, 4, ambient=0.5)
+    out = [[], []]
+
+    def work(k):
+        c = api.Context(0)
+        try:
+            for _ in range(6):
+                out[k].append(render(c, scenes[k], o)[0])
+        finally:
+            c.close()
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    [t.start() for t in th]
+    [t.join() for t in th]
+    for k in range(2):
+        c = api.Context(0)
+        want = render(c, scenes[k], o)[0]
+        c.close()
+        assert len(out[k]) == 6 and all(np.array_equal(x, want) for x in out[k])
