@@ -66,8 +66,8 @@ PT_API pt_status pt_set_traversal(pt_context *ctx, uint32_t threads, uint32_t cl
  * time, 1 the default (three arenas, or the scene class's tuned count), 2
  * or 3 that many arenas. Images are identical whatever the setting. */
 PT_API pt_status pt_set_wave_overlap(pt_context *ctx, int on);
-/* Occupancy of the wavefront shade kernel: 3 (default) or 4 blocks of 128
- * threads per SM. Images are identical either way. */
+/* Occupancy of the shade kernel of layered materials: 3 (default) or 4 times
+ * 128 threads per SM. Images are identical either way. */
 PT_API pt_status pt_set_shade_blocks(pt_context *ctx, uint32_t blocks_per_sm);
 /* Wavefront waves replayed from CUDA graphs (one capture per bounce count
  * and sort setting; on by default, bypassed while stage timing is on). */
@@ -90,7 +90,7 @@ typedef struct pt_tune_choice {
   uint32_t material_sort;        /* 0 / 1 */
   uint32_t wave_slots;
   float samples_per_s;           /* calibration throughput */
-  uint32_t shade_blocks_per_sm;  /* 3 or 4: the shade kernel's occupancy */
+  uint32_t shade_blocks_per_sm;  /* 3 or 4: the layered shade kernel's occupancy */
   uint32_t wave_arenas;          /* 2 or 3: overlapped waves in flight (pt_set_wave_overlap) */
   uint32_t traversal_threads;    /* 128 or 256: block size of the traversal kernels (pt_set_traversal) */
   uint32_t claim_chunk;          /* 1, 2 or 4: queue entries a traversal lane claims per refill */
@@ -183,7 +183,7 @@ PT_API pt_status pt_set_schedule(pt_context *ctx, uint32_t schedule);
 PT_API pt_status pt_set_wave_slots(pt_context *ctx, uint32_t slots);
 /* BVH node layout the wavefront's traversal kernels walk, for extension and
  * for shadow rays: 2 (two-child 64-byte nodes) or 4 (the same tree as
- * four-child 128-byte nodes). Default: 4 for both. Hits are identical
+ * four-child quantised 64-byte nodes). Default: 4 for both. Hits are identical
  * either way. */
 PT_API pt_status pt_set_node_width(pt_context *ctx, uint32_t extension_width, uint32_t shadow_width);
 /* Device time in ms of the last refine's path-tracing kernels (CUDA events

@@ -149,7 +149,8 @@ class Context:
         self.check(self.lib.pt_set_wave_overlap(self.ptr, int(on)))
 
     def set_shade_blocks(self, blocks_per_sm: int) -> None:
-        """Occupancy of the wavefront shade kernel (3 or 4 blocks per SM)."""
+        """Occupancy of the layered materials' shade kernel (3 or 4 times 128
+        threads per SM)."""
         self.check(self.lib.pt_set_shade_blocks(self.ptr, int(blocks_per_sm)))
 
     def set_traversal(self, threads: int = 256, claim_chunk: int = 1) -> None:

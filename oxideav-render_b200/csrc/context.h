@@ -20,7 +20,7 @@ namespace ptd {
 struct TuneChoice {
   uint32_t schedule, wide_nodes, material_sort, wave_slots;
   float samples_per_s;
-  uint32_t shade_blocks = 3;  // k_wf_shade blocks per SM (3 or 4)
+  uint32_t shade_blocks = 3;  // layered k_wf_shade: 3 or 4 times 128 threads per SM
   uint32_t arenas = 2;        // overlapped waves in flight (2 or 3)
   uint32_t trav_threads = 256;  // traversal kernels' block size (128 or 256)
   uint32_t claim_chunk = 1;     // queue entries per traversal refill (1, 2, 4)
@@ -46,7 +46,7 @@ struct pt_context {
   // (default: both kinds).
   uint32_t wide_nodes = ptd::WIDE_EXTENSION | ptd::WIDE_SHADOW;
   bool material_sort = true;  // bucket each shade queue by material
-  uint32_t shade_blocks = 3;   // k_wf_shade instantiation: blocks per SM (3 or 4)
+  uint32_t shade_blocks = 3;   // layered k_wf_shade: 3 or 4 times 128 threads per SM
   uint32_t trav_threads = 256;  // traversal kernels' block size (128 or 256; 1,024 threads per SM)
   uint32_t claim_chunk = 1;     // queue entries a traversal lane claims per refill (1, 2 or 4)
   int bvh_builder = ptd::BVH_BUILD_AUTO;  // where pt_scene_upload builds the BVH (ptd::BvhBuilder)
