@@ -361,7 +361,7 @@ pt_status run_jobs(pt_context *ctx, std::vector<pt_tracer *> &tracers, std::vect
   CK(ctx, cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), ctx->stream));
   StageTimer timer;
   if (ctx->stage_timing) {
-    size_t need = waves.size() * (4 * (size_t)max_iter + 3) + 1;
+    const size_t need = waves.size() * wave_marks(max_iter) + 1;  // and the end
     while (ctx->stage_events.size() < need) {
       cudaEvent_t ev;
       CK(ctx, cudaEventCreate(&ev));
@@ -431,6 +431,8 @@ pt_status run_jobs(pt_context *ctx, std::vector<pt_tracer *> &tracers, std::vect
   ctx->last_batch_rays = c.ext_rays + c.shadow_rays;
   if (c.error_flags & ERR_STACK_OVERFLOW) return fail(ctx, PT_ERR_DEVICE, "BVH traversal stack overflow");
   for (size_t j = 0; j < jobs.size(); ++j) tracers[j]->samples += jobs[j].target;
+  if (timer.error != cudaSuccess)
+    return fail(ctx, PT_ERR_DEVICE, std::string("stage timing is incomplete: ") + cudaGetErrorString(timer.error));
   return PT_OK;
 }
 

@@ -10,18 +10,25 @@
 namespace ptd {
 
 // Optional per-stage CUDA events: mark(kind) records the next event of a
-// caller-owned pool on the stream; consecutive events bracket one stage.
+// caller-owned pool on the stream; consecutive events bracket one stage. A
+// mark that has no event left, or whose record fails, ends the recording
+// with `error` set: stage times then miss whatever came after.
 struct StageTimer {
   cudaEvent_t *events = nullptr;
   size_t capacity = 0;
+  cudaError_t error = cudaSuccess;
   std::vector<int> kinds;
   size_t count() const { return kinds.size(); }
   void mark(int kind, cudaStream_t st) {
-    if (!events || kinds.size() >= capacity) return;
-    cudaEventRecord(events[kinds.size()], st);
-    kinds.push_back(kind);
+    if (!events || error != cudaSuccess) return;
+    error = kinds.size() < capacity ? cudaEventRecord(events[kinds.size()], st) : cudaErrorInvalidValue;
+    if (error == cudaSuccess) kinds.push_back(kind);
   }
 };
+// The most marks a wave of `iterations` bounces makes: extend, sort, light
+// sampling, shade and shadow each bounce, ray generation and accumulate
+// (launch_wavefront; the megakernel makes two).
+constexpr size_t wave_marks(uint32_t iterations) { return 5 * (size_t)iterations + 2; }
 
 cudaError_t set_tables(const float *sheen_lut, const float *srgb_thresh);
 cudaError_t launch_megakernel(const DevRequest *reqs, const WaveSegment *segs, uint32_t nseg, uint32_t total,
