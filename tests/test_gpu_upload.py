@@ -2,6 +2,9 @@
 change hands (64 triangles is its least, subtrees of at most 32 go to a warp,
 tiles of 1,024), with coinciding, flat and NaN triangles, against the host
 build; and the context's memory pool over many uploads and two threads."""
+import os
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -97,6 +100,7 @@ def test_two_contexts_in_two_threads():
     def work(k):
         c = api.Context(0)
         try:
+            c.set_schedule(abi.PT_SCHEDULE_WAVEFRONT)  # of itself so small a refine is the megakernel's
             for _ in range(6):
                 out[k].append(render(c, scenes[k], o)[0])
         finally:
@@ -107,6 +111,51 @@ def test_two_contexts_in_two_threads():
     [t.join() for t in th]
     for k in range(2):
         c = api.Context(0)
+        c.set_schedule(abi.PT_SCHEDULE_WAVEFRONT)
         want = render(c, scenes[k], o)[0]
         c.close()
         assert len(out[k]) == 6 and all(np.array_equal(x, want) for x in out[k])
+
+
+FIRST_WAVES = """
+import sys, threading, time
+sys.path.insert(0, {root!r})
+import __graft_entry__ as entry
+entry.load_package()
+import numpy as np
+from oxideav_render_b200 import abi, api, testscenes as ts
+scene, o = ts.sphere_grid(3, 2, 12, 6), ts.pt_opts(48, 1, 3, ambient=0.5)
+N, out, failed = 8, [None] * 8, []
+ready = threading.Barrier(N)
+
+def work(k):
+    try:
+        c = api.Context(0)
+        c.set_schedule(abi.PT_SCHEDULE_WAVEFRONT)
+        c.set_traversal((256, 128)[k % 2], 1)
+        t = api.PathTracer(c)
+        t.sync(scene, o)
+        ready.wait(60)
+        time.sleep(k * {step})
+        t.refine(1)
+        out[k] = t.accum()
+    except Exception as e:
+        failed.append(repr(e))
+
+th = [threading.Thread(target=work, args=(k,)) for k in range(N)]
+[t.start() for t in th]
+[t.join() for t in th]
+assert not failed, failed
+assert all(np.array_equal(a, out[0]) for a in out)
+print("whole")
+"""
+
+
+@pytest.mark.parametrize("step", [0.0, 1e-4, 1e-3])
+def test_first_waves_of_several_threads(step):
+    """A process's first waves, started by eight contexts a little apart: the
+    grid sizes are looked up while the others already launch."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", FIRST_WAVES.format(root=root, step=step)], capture_output=True,
+                       text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "whole", r.stderr[-2000:]
