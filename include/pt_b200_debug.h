@@ -171,6 +171,11 @@ PT_API pt_status pt_debug_scene_texels(pt_context *ctx, uint32_t scene_id, float
  * fail with PT_ERR_OOM as if cudaMalloc had run out of memory, without
  * calling CUDA. The context stays usable. 0 disarms it. */
 PT_API pt_status pt_debug_fail_allocations(pt_context *ctx, uint32_t count);
+/* The memory pool that the context's scenes come from, once its stream is
+ * idle: bytes taken from the device, and bytes of those in use. The rest is
+ * kept for later uploads, up to 1 GiB, and given back when the context is
+ * destroyed or an allocation of any context on the device fails. */
+PT_API pt_status pt_debug_pool_bytes(pt_context *ctx, uint64_t bytes[2]);
 
 /* Schedule of the hot loop: one path per thread (megakernel), or the
  * wavefront (extend / shade / shadow kernels over compacted queues; the

@@ -19,7 +19,7 @@ from __future__ import annotations
 
 import ctypes as C
 import weakref
-from typing import Optional
+from typing import Optional, Tuple
 
 import numpy as np
 
@@ -166,6 +166,13 @@ class Context:
         """pt_debug_fail_allocations: the next `count` device allocations of
         the context fail with PT_ERR_OOM (host-side injection, no CUDA call)."""
         self.check(self.lib.pt_debug_fail_allocations(self.ptr, int(count)))
+
+    def pool_bytes(self) -> Tuple[int, int]:
+        """pt_debug_pool_bytes: bytes the context's memory pool holds of the
+        device, and bytes of those in use."""
+        v = np.zeros(2, np.uint64)
+        self.check(self.lib.pt_debug_pool_bytes(self.ptr, v.ctypes.data_as(native.u64p)))
+        return int(v[0]), int(v[1])
 
     def set_stage_timing(self, on: bool) -> None:
         self.check(self.lib.pt_set_stage_timing(self.ptr, 1 if on else 0))

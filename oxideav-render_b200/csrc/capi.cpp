@@ -45,20 +45,24 @@ pt_status fail(pt_context *ctx, pt_status st, const std::string &msg) {
                   std::string(#call) + ": " + cudaGetErrorString(e_));                           \
   } while (0)
 
-// Consumes one injected allocation failure of `ctx`, if armed.
+// Consumes one injected allocation failure of `ctx`, if armed: one that the
+// pools' cached memory, given back first as for any other, did not help.
 bool injected_oom(pt_context *ctx) {
   if (!ctx) return false;
   uint32_t n = ctx->fail_allocs.load();
   while (n > 0)
-    if (ctx->fail_allocs.compare_exchange_weak(n, n - 1)) return true;
+    if (ctx->fail_allocs.compare_exchange_weak(n, n - 1)) {
+      trim_pools();
+      return true;
+    }
   return false;
 }
 
-// cudaMalloc, or the injected out-of-memory failure.
+// cudaMalloc by way of device_malloc, or the injected out-of-memory failure.
 template <class T>
 cudaError_t dev_malloc(pt_context *ctx, T **p, size_t bytes) {
   if (injected_oom(ctx)) return cudaErrorMemoryAllocation;
-  return cudaMalloc(p, bytes);
+  return device_malloc((void **)p, bytes);
 }
 
 template <class F>
@@ -521,7 +525,7 @@ pt_status autotune_scene(pt_context *ctx, const pt_tracer *t, SceneHost *sc, con
   s.have_state = true;
   s.dirty = false;
   const size_t n = (size_t)s.w * s.h * 4;
-  CK(ctx, cudaMalloc(&s.d_accum, n * sizeof(double)));
+  CK(ctx, device_malloc((void **)&s.d_accum, n * sizeof(double)));
   s.accum_cap = n;
   struct Free {
     double *p;
@@ -834,7 +838,7 @@ pt_status engine_create(int device, pt_context **out) {
   host_sheen_lut(sheen);
   host_srgb_thresholds(thr);
   if (e == cudaSuccess) e = set_tables(sheen, thr);
-  if (e == cudaSuccess) e = cudaMalloc(&ctx->d_ctr, sizeof(DevCounters));
+  if (e == cudaSuccess) e = device_malloc((void **)&ctx->d_ctr, sizeof(DevCounters));
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev1);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
@@ -846,7 +850,10 @@ pt_status engine_create(int device, pt_context **out) {
     props.location.id = device;
     uint64_t keep = pt_context::kPoolKeep;
     if (cudaMemPoolCreate(&ctx->pool, &props) != cudaSuccess) ctx->pool = nullptr;
-    if (ctx->pool) cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (ctx->pool) {
+      cudaMemPoolSetAttribute(ctx->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      register_pool(device, ctx->pool, ctx->stream);
+    }
     cudaGetLastError();
   }
   if (e != cudaSuccess) {
@@ -895,7 +902,10 @@ void pt_destroy(pt_context *ctx) {
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-  if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
+  if (ctx->pool) {
+    unregister_pool(ctx->pool);
+    cudaMemPoolDestroy(ctx->pool);
+  }
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   ctx->staging.release();
   delete ctx;
@@ -1419,6 +1429,17 @@ pt_status pt_debug_fail_allocations(pt_context *ctx, uint32_t count) {
   return PT_OK;
 }
 
+pt_status pt_debug_pool_bytes(pt_context *ctx, uint64_t bytes[2]) {
+  if (!ctx || !bytes) return fail(ctx, PT_ERR_INVALID_ARG, "NULL argument");
+  bytes[0] = bytes[1] = 0;
+  if (!ctx->pool) return PT_OK;
+  CK(ctx, cudaSetDevice(ctx->device));
+  CK(ctx, cudaStreamSynchronize(ctx->stream));
+  CK(ctx, cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &bytes[0]));
+  CK(ctx, cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &bytes[1]));
+  return PT_OK;
+}
+
 pt_status pt_set_wave_graphs(pt_context *ctx, int on) {
   if (!ctx) return fail(ctx, PT_ERR_INVALID_ARG, "context is NULL");
   ctx->use_graphs = on != 0;
@@ -1474,7 +1495,7 @@ pt_status pt_debug_sobol(pt_context *ctx, uint32_t n, uint32_t seed, float *out)
     if (n == 0) return PT_OK;
     CK(ctx, cudaSetDevice(ctx->device));
     float4 *d = nullptr;
-    CK(ctx, cudaMalloc(&d, (size_t)n * sizeof(float4)));
+    CK(ctx, device_malloc((void **)&d, (size_t)n * sizeof(float4)));
     cudaError_t e = launch_debug_sobol(n, seed, d, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, d, (size_t)n * sizeof(float4), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
@@ -1496,7 +1517,7 @@ pt_status pt_debug_pattern(pt_tracer *t, uint32_t index, uint32_t pattern, float
     CK(ctx, cudaMemcpyAsync(t->d_req, &rq, sizeof rq, cudaMemcpyHostToDevice, ctx->stream));
     uint32_t npix = t->w * t->h;
     float4 *d = nullptr;
-    CK(ctx, cudaMalloc(&d, (size_t)npix * sizeof(float4)));
+    CK(ctx, device_malloc((void **)&d, (size_t)npix * sizeof(float4)));
     cudaError_t e = launch_debug_pattern(t->d_req, npix, index, pattern, d, ctx->stream);
     if (e == cudaSuccess)
       e = cudaMemcpyAsync(out, d, (size_t)npix * sizeof(float4), cudaMemcpyDeviceToHost, ctx->stream);
@@ -1520,8 +1541,8 @@ pt_status pt_debug_primary_hits(pt_tracer *t, uint32_t index, uint32_t *out_g, f
     uint32_t npix = t->w * t->h;
     uint32_t *dg = nullptr;
     float4 *dt = nullptr;
-    CK(ctx, cudaMalloc(&dg, (size_t)npix * 4));
-    cudaError_t e = cudaMalloc(&dt, (size_t)npix * sizeof(float4));
+    CK(ctx, device_malloc((void **)&dg, (size_t)npix * 4));
+    cudaError_t e = device_malloc((void **)&dt, (size_t)npix * sizeof(float4));
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_ctr, 0, sizeof(DevCounters), ctx->stream);
     if (e == cudaSuccess) e = launch_debug_primary(t->d_req, npix, index, dg, dt, ctx->d_ctr, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out_g, dg, (size_t)npix * 4, cudaMemcpyDeviceToHost, ctx->stream);
@@ -1543,7 +1564,7 @@ pt_status pt_debug_bsdf(pt_context *ctx, const float *params, const float *dirs,
     CK(ctx, cudaSetDevice(ctx->device));
     float *d = nullptr;
     size_t fl = 43 + 3 * (size_t)n + 3 * (size_t)n + 12 * (size_t)n;
-    CK(ctx, cudaMalloc(&d, fl * 4));
+    CK(ctx, device_malloc((void **)&d, fl * 4));
     float *dp = d, *dd = d + 43, *du = dd + 3 * (size_t)n, *dout = du + 3 * (size_t)n;
     cudaError_t e = cudaMemcpyAsync(dp, params, 43 * 4, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dd, dirs, 12 * (size_t)n, cudaMemcpyHostToDevice, ctx->stream);

@@ -52,7 +52,8 @@ struct pt_context {
   int bvh_builder = ptd::BVH_BUILD_AUTO;  // where pt_scene_upload builds the BVH (ptd::BvhBuilder)
   // Device memory of scenes, trees, build scratch and raycast frames: a
   // one-shot render takes and returns some 70 MB, which the pool keeps (up to
-  // kPoolKeep; returned with the context) instead of unmapping at every
+  // kPoolKeep; returned with the context, or as soon as an allocation of any
+  // context on the device fails: device_mem.h) instead of unmapping at every
   // release. Every allocation is made, used and freed on `stream`, or between
   // synchronisations with it. nullptr where the device has no pools.
   cudaMemPool_t pool = nullptr;

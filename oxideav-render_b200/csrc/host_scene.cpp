@@ -1124,16 +1124,6 @@ void emit_tree(const std::vector<BNode> &in_nodes, const std::vector<uint32_t> &
 }  // namespace
 
 // ============================================================ arena
-cudaError_t device_alloc(void **p, uint64_t bytes, cudaStream_t stream, cudaMemPool_t pool) {
-  if (!pool) return stream ? cudaMallocAsync(p, bytes, stream) : cudaMalloc(p, bytes);
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, stream);
-  if (e != cudaErrorMemoryAllocation) return e;
-  cudaGetLastError();
-  cudaStreamSynchronize(stream);
-  cudaMemPoolTrimTo(pool, 0);
-  return cudaMallocFromPoolAsync(p, bytes, pool, stream);
-}
-
 void DeviceArena::release() {
   if (base) {
     if (stream)
@@ -1163,7 +1153,7 @@ struct ArenaPlan {
 
 std::string commit(ArenaPlan &plan, DeviceArena &arena, bool &oom, cudaStream_t stream) {
   if (plan.total == 0) plan.total = 256;
-  cudaError_t e = stream ? cudaMallocAsync(&arena.base, plan.total, stream) : cudaMalloc(&arena.base, plan.total);
+  cudaError_t e = device_alloc(&arena.base, plan.total, stream, nullptr);
   if (e != cudaSuccess) {
     oom = e == cudaErrorMemoryAllocation;
     arena.base = nullptr;

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "dev_types.h"
+#include "device_mem.h"
 
 namespace ptd {
 
@@ -38,12 +39,6 @@ void build_bvh_spatial(const float *pos, uint32_t tri_count, const uint32_t *rec
 // One device allocation holding a scene (or an environment) plus the
 // device copy of its descriptor. `stream` non-null: the allocation is
 // stream-ordered (cudaMallocAsync) and is freed in that stream's order.
-// Device memory for scenes, their trees and build scratch: from `pool`
-// (stream-ordered; the context's, see pt_context::pool), else from the
-// device's default pool on `stream`, else synchronously. A pool that cannot
-// serve the request gives its cached memory back first and is asked again.
-cudaError_t device_alloc(void **p, uint64_t bytes, cudaStream_t stream, cudaMemPool_t pool);
-
 struct DeviceArena {
   void *base = nullptr;
   uint64_t bytes = 0;

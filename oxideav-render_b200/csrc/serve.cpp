@@ -236,7 +236,10 @@ enum class Admit { Yes, Wait, Failed };
 bool injected_oom(pt_server *s) {
   uint32_t n = s->fail_allocs.load();
   while (n > 0)
-    if (s->fail_allocs.compare_exchange_weak(n, n - 1)) return true;
+    if (s->fail_allocs.compare_exchange_weak(n, n - 1)) {
+      trim_pools();
+      return true;
+    }
   return false;
 }
 
@@ -386,7 +389,7 @@ Admit try_admit(pt_server *s, const std::shared_ptr<Request> &r, std::unique_loc
   pt_tracer &t = acc.t;
   if (!t.d_accum) {
     size_t bytes = (size_t)t.w * t.h * 4 * sizeof(double);
-    cudaError_t e = injected_oom(s) ? cudaErrorMemoryAllocation : cudaMallocAsync((void **)&t.d_accum, bytes, stream);
+    cudaError_t e = injected_oom(s) ? cudaErrorMemoryAllocation : device_alloc((void **)&t.d_accum, bytes, stream, nullptr);
     if (e == cudaSuccess) e = cudaMemsetAsync(t.d_accum, 0, bytes, stream);
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -442,7 +445,7 @@ cudaError_t grow_pair(T *&d, T *&h, size_t &cap, size_t need) {
   d = nullptr;
   h = nullptr;
   cap = 0;
-  cudaError_t e = cudaMalloc((void **)&d, n * sizeof(T));
+  cudaError_t e = device_malloc((void **)&d, n * sizeof(T));
   if (e == cudaSuccess) e = cudaMallocHost((void **)&h, n * sizeof(T));
   if (e == cudaSuccess) cap = n;
   return e;
@@ -566,7 +569,7 @@ void launch_next_wave(pt_server *s) {
       if (s->d_resolve) cudaFreeAsync(s->d_resolve, stream);
       s->d_resolve = nullptr;
       s->resolve_cap = 0;
-      e = cudaMallocAsync((void **)&s->d_resolve, npix * sizeof(float4), stream);
+      e = device_alloc((void **)&s->d_resolve, npix * sizeof(float4), stream, nullptr);
       if (e == cudaSuccess) s->resolve_cap = npix;
     }
     r->hdr_bytes = npix * sizeof(float4);

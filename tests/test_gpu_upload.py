@@ -1,7 +1,8 @@
 """Scene uploads: the device binned-SAH build at the sizes where its kernels
 change hands (64 triangles is its least, subtrees of at most 32 go to a warp,
 tiles of 1,024), with coinciding, flat and NaN triangles, against the host
-build; and the context's memory pool over many uploads and two threads."""
+build; the context's memory pool: its reuse, its limit, and that failing
+allocations give its cache back; and contexts in several threads."""
 import os
 import subprocess
 import sys
@@ -64,14 +65,12 @@ def test_device_build_equals_the_host_build(ctx, kind, n):
         assert sa["sah_cost"] == pytest.approx(sb["sah_cost"], rel=1e-9)
 
 
-def test_pool_keeps_a_bounded_cache():
-    import torch
+def test_uploads_and_releases_reuse_the_pool():
     scene, o = cloud("random", 50000), ts.pt_opts(16, 1, 2, ambient=0.5)
     c = api.Context(0)
     try:
         d = scene.to_desc(o)
-        want = None
-        ids = []
+        want, ids, one = None, [], 0
         for k in range(40):
             ids.append(c.upload(d))
             if k % 3:
@@ -80,16 +79,74 @@ def test_pool_keeps_a_bounded_cache():
                 got = render(c, scene, o)[0]
                 want = got if want is None else want
                 assert np.array_equal(got, want)
-        held = torch.cuda.mem_get_info()[0]
-        for i in ids:
-            c.release(i)
-        # Released scenes stay in the pool up to its limit, no further.
-        big = ts.stress_c2(64, 64, 1, grid=512, spheres=50)[0].to_desc(o)
-        for _ in range(3):
-            c.release(c.upload(big))
-        assert held - torch.cuda.mem_get_info()[0] < 3 << 29
+            if k == 0:
+                one = c.pool_bytes()[1]
+        # 14 scenes stay; the 26 released ones made room for others and for
+        # what the builds and renders took and returned.
+        reserved, used = c.pool_bytes()
+        assert len(ids) == 14 and used == 14 * one and reserved <= used + 6 * one + (128 << 20)
     finally:
         c.close()
+
+
+def test_pool_keeps_at_most_a_gigabyte():
+    big = ts.stress_c2(64, 64, 1, grid=384, spheres=50)[0].to_desc(ts.pt_opts(16, 1, 2))
+    c = api.Context(0)
+    try:
+        ids, keep = [], 1 << 30
+        while c.pool_bytes()[1] < 2 * keep and len(ids) < 40:
+            ids.append(c.upload(big))
+        one = c.pool_bytes()[1] // len(ids)
+        assert c.pool_bytes()[1] >= 2 * keep and one < keep // 4
+        for i in ids:
+            c.release(i)
+        # What is over the limit goes back in whole blocks of the pool, at the
+        # next synchronisation: nothing like the 2 GiB that were in use.
+        reserved, used = c.pool_bytes()
+        assert used == 0 and one <= reserved <= keep + one
+        # The cache serves the next upload.
+        c.upload(big)
+        assert c.pool_bytes()[0] <= reserved + one
+    finally:
+        c.close()
+
+
+@pytest.mark.parametrize("which", ["upload", "refit", "accumulator", "wave arena", "another context"])
+def test_a_failing_allocation_gives_the_cache_back(which):
+    scene, o = cloud("random", 300000), ts.pt_opts(24, 2, 3, ambient=0.5)
+    c, other = api.Context(0), api.Context(0)
+    try:
+        c.set_schedule(abi.PT_SCHEDULE_WAVEFRONT)
+        d = scene.to_desc(o)
+        kept = c.upload(d)
+        used = c.pool_bytes()[1]
+        gone = [c.upload(d) for _ in range(8)]
+        for i in gone:
+            c.release(i)
+        assert c.pool_bytes()[0] >= used + (192 << 20) and c.pool_bytes()[1] == used
+        t = api.PathTracer(c)
+        if which == "wave arena":
+            t.sync_resident(kept, scene, o)
+        failing = other if which == "another context" else c
+        failing.fail_allocations(1)
+        with pytest.raises(api.RenderError) as e:
+            if which == "refit":
+                c.refit(kept, d)
+            elif which == "accumulator":
+                t.sync_resident(kept, scene, o)
+            elif which == "wave arena":
+                t.refine(2)
+            else:
+                failing.upload(d)
+        assert e.value.status == abi.PT_ERR_OOM
+        reserved, now = c.pool_bytes()
+        assert now == used and reserved <= used + (64 << 20)  # whole blocks of the pool
+        # Both contexts go on.
+        a, b = render(c, scene, o)[0], render(other, scene, o)[0]
+        assert np.array_equal(a, b)
+    finally:
+        c.close()
+        other.close()
 
 
 def test_two_contexts_in_two_threads():
