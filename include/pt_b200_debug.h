@@ -37,7 +37,8 @@ PT_API pt_status pt_tracer_traversal_split(const pt_tracer *tr, uint64_t out[4])
 /* Per-stage device time of refine calls (CUDA events between the kernels of
  * each stage on the context stream), off by default. Stages, in order:
  * ray generation, closest hit, shade, shadow rays, accumulate, megakernel,
- * material sort. */
+ * material sort, light sampling. While on, waves run one at a time without
+ * graphs, and small refines stay on the wavefront. */
 PT_API pt_status pt_set_stage_timing(pt_context *ctx, int on);
 PT_API pt_status pt_tracer_stage_ms(const pt_tracer *tr, float *out, uint32_t n);
 /* The same figures for the last refine or batch of the context as a whole
@@ -48,6 +49,8 @@ PT_API pt_status pt_tracer_stage_ms(const pt_tracer *tr, float *out, uint32_t n)
  * per-stage device ms (stage timing on). */
 PT_API pt_status pt_batch_counters(const pt_context *ctx, uint64_t out[9]);
 PT_API pt_status pt_batch_stage_ms(const pt_context *ctx, float *out, uint32_t n);
+/* The schedule (pt_schedule) that the last refine or batch ran on. */
+PT_API pt_status pt_batch_schedule(const pt_context *ctx, uint32_t *schedule);
 /* Wavefront shade order: nonzero buckets the active queue by (scene,
  * material) before each shade launch so warps shade one material at a time
  * (three small kernels per bounce; on by default). Images are identical

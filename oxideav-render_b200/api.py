@@ -430,6 +430,13 @@ def batch_counters(ctx: Context) -> dict:
     return out
 
 
+def batch_schedule(ctx: Context) -> int:
+    """pt_batch_schedule: the schedule the last refine or batch ran on."""
+    v = C.c_uint32()
+    ctx.check(ctx.lib.pt_batch_schedule(ctx.ptr, C.byref(v)))
+    return v.value
+
+
 def batch_stats(ctx: Context) -> dict:
     ms, waves, rays = C.c_float(), C.c_uint32(), C.c_uint64()
     ctx.check(ctx.lib.pt_batch_stats(ctx.ptr, C.byref(ms), C.byref(waves), C.byref(rays)))

@@ -398,6 +398,7 @@ pt_status run_jobs(pt_context *ctx, std::vector<pt_tracer *> &tracers, std::vect
   CK(ctx, cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
   ctx->last_batch_ms = ms;
   ctx->last_batch_waves = (uint32_t)waves.size();
+  ctx->last_batch_schedule = ctx->schedule;
   {
     uint64_t samples = 0, rounds = 0;
     for (const Job &jb : jobs) samples += (uint64_t)jb.npix * jb.target;
@@ -1080,6 +1081,12 @@ pt_status pt_batch_stats(const pt_context *ctx, float *ms, uint32_t *waves, uint
 pt_status pt_batch_counters(const pt_context *ctx, uint64_t out[9]) {
   if (!ctx || !out) return fail(nullptr, PT_ERR_INVALID_ARG, "NULL argument");
   std::memcpy(out, ctx->last_batch_counts, sizeof ctx->last_batch_counts);
+  return PT_OK;
+}
+
+pt_status pt_batch_schedule(const pt_context *ctx, uint32_t *schedule) {
+  if (!ctx || !schedule) return fail(nullptr, PT_ERR_INVALID_ARG, "NULL argument");
+  *schedule = ctx->last_batch_schedule;
   return PT_OK;
 }
 

@@ -71,6 +71,7 @@ struct pt_context {
   size_t req_cap = 0;
   float last_batch_ms = 0.0f;
   uint32_t last_batch_waves = 0;
+  uint32_t last_batch_schedule = PT_SCHEDULE_WAVEFRONT;  // that the last refine or batch ran on
   uint64_t last_batch_rays = 0;
   // Counters of the last batch: extension / shadow rays, their nodes and
   // triangles, samples, waves (pt_batch_counters); per-stage ms.

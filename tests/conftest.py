@@ -28,7 +28,10 @@ def pt():
 
 @pytest.fixture(scope="session")
 def ctx():
-    from oxideav_render_b200 import api
+    """A context on the wavefront. One whose schedule nobody chose runs small
+    refines on the megakernel: tests of that make their own."""
+    from oxideav_render_b200 import abi, api
     c = api.Context(0)
+    c.set_schedule(abi.PT_SCHEDULE_WAVEFRONT)
     yield c
     c.close()

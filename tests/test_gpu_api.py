@@ -253,14 +253,19 @@ def test_scene_release_and_counts(ctx):
 
 def test_a_fresh_context_runs_the_wavefront_by_default():
     # The drop-in path (make_renderer / pt_create with nothing set) must run
-    # the wavefront schedule, and its accumulator must equal the megakernel's.
-    scene, opts = ts.sphere_grid_c1(64, 4)
+    # the wavefront schedule, of itself beyond small refines and at any size
+    # once stage times are asked for, and its accumulator must equal the
+    # megakernel's.
+    scene, opts = ts.sphere_grid_c1(256, 4)
     fresh = api.Context(0)
     try:
-        fresh.set_stage_timing(True)  # only records per-stage device times
         t = api.PathTracer(fresh)
         t.sync(scene, opts)
-        t.refine(4)
+        t.refine(3)  # 196,608 paths
+        assert api.batch_schedule(fresh) == abi.PT_SCHEDULE_WAVEFRONT
+        fresh.set_stage_timing(True)
+        t.refine(1)
+        assert api.batch_schedule(fresh) == abi.PT_SCHEDULE_WAVEFRONT
         stages = t.stage_ms()
         assert stages["extend"] > 0.0 and stages["shade"] > 0.0 and stages["shadow"] > 0.0, stages
         assert stages["megakernel"] == 0.0, stages
@@ -274,6 +279,7 @@ def test_a_fresh_context_runs_the_wavefront_by_default():
         t = api.PathTracer(mk)
         t.sync(scene, opts)
         t.refine(4)
+        assert api.batch_schedule(mk) == abi.PT_SCHEDULE_MEGAKERNEL
         assert np.array_equal(t.accum(), wf)
         t.close()
     finally:

@@ -14,7 +14,7 @@ import math
 import numpy as np
 import pytest
 
-from oxideav_render_b200 import api, testscenes as ts
+from oxideav_render_b200 import abi, api, testscenes as ts
 from oxideav_render_b200.options import LightStrategy, PathTraceOptions
 from oxideav_render_b200.scene import Camera
 
@@ -22,6 +22,15 @@ pytestmark = pytest.mark.gpu
 
 MAE_MAX = 2e-3
 PSNR_MIN = 45.0
+
+
+@pytest.fixture(scope="module", params=[abi.PT_SCHEDULE_WAVEFRONT, abi.PT_SCHEDULE_MEGAKERNEL],
+                ids=["wavefront", "megakernel"])
+def ctx(request):
+    c = api.Context(0)
+    c.set_schedule(request.param)
+    yield c
+    c.close()
 
 
 def oracle_tracer(oracle, scene, opts, env=None):

@@ -1,13 +1,14 @@
 """Small refines: a context whose schedule nobody chose runs them on the
 megakernel up to a size that depends on area lights; the accumulator and the
 ray counts are those of the wavefront on both sides of each limit, alone and
-in a batch, and over several calls."""
+in a batch, and over several calls. Which schedule ran is asked, not assumed."""
 import numpy as np
 import pytest
 
 from oxideav_render_b200 import abi, api, testscenes as ts
 
 pytestmark = pytest.mark.gpu
+W, M = abi.PT_SCHEDULE_WAVEFRONT, abi.PT_SCHEDULE_MEGAKERNEL
 
 
 def render(fixed, scene, opts, calls, env=None):
@@ -19,11 +20,12 @@ def render(fixed, scene, opts, calls, env=None):
         if env is not None:
             t.set_environment(api.EnvironmentMap(env))
         t.sync(scene, opts)
-        rays = []
+        rays, schedules = [], []
         for n in calls:
             t.refine(n)
             rays.append(t.ray_counts())
-        return t.accum(), rays, t.samples()
+            schedules.append(api.batch_schedule(c))
+        return t.accum(), rays, t.samples(), schedules
     finally:
         c.close()
 
@@ -33,9 +35,12 @@ def render(fixed, scene, opts, calls, env=None):
 def test_small_refines_equal_the_wavefront(lit, width, height):
     scene = ts.cornell_c0()[0] if lit else ts.sphere_grid(3, 2, 12, 6)
     o = ts.pt_opts(width, 1, 5, h=height, ambient=0.3)
-    a, ra, na = render(False, scene, o, (1, 1, 2))
-    b, rb, nb = render(True, scene, o, (1, 1, 2))
+    calls = (1, 1, 2)
+    a, ra, na, sa = render(False, scene, o, calls)
+    b, rb, nb, sb = render(True, scene, o, calls)
     assert np.array_equal(a, b) and ra == rb and na == nb == 4
+    limit = (24 if lit else 96) << 10
+    assert sa == [M if n * width * height <= limit else W for n in calls] and sb == [W, W, W]
 
 
 def test_small_batch_equals_the_wavefront():
@@ -52,6 +57,7 @@ def test_small_batch_equals_the_wavefront():
                 t.sync(s, ts.pt_opts(31 + k, 2, 4, h=17, seed=k, ambient=0.2))
                 tr.append(t)
             api.refine_many(c, tr, [2, 1, 3])
+            assert api.batch_schedule(c) == (W if fixed else M)
             out.append([t.accum() for t in tr])
         finally:
             c.close()
