@@ -182,9 +182,10 @@ PT_API pt_status pt_debug_pool_bytes(pt_context *ctx, uint64_t bytes[2]);
 
 /* Schedule of the hot loop: one path per thread (megakernel), or the
  * wavefront (extend / shade / shadow kernels over compacted queues; the
- * default of a new context, which runs refines of a few thousand paths on the
- * megakernel until this or another setting of the wavefront is called). Both
- * produce bit-identical accumulators. */
+ * default of a new context, which runs refines of up to 64 K paths on the
+ * megakernel where that is the faster one, until this or another setting of
+ * the wavefront is called, its default value included, or the scene's class
+ * is tuned). Both produce bit-identical accumulators. */
 typedef enum pt_schedule { PT_SCHEDULE_MEGAKERNEL = 0, PT_SCHEDULE_WAVEFRONT = 1 } pt_schedule;
 PT_API pt_status pt_set_schedule(pt_context *ctx, uint32_t schedule);
 /* Maximum path slots per wave (device sample buffer 16 B per slot). */

@@ -149,6 +149,8 @@ Job make_job(const pt_tracer &t, const SceneHost &sc, const EnvHost *env, uint32
   j.iterations = t.opts.path_trace.max_bounces + 1;
   j.shadow_slots = sc.light_count + 1;
   j.scene_key = t.scene_id;
+  j.lit_lights = sc.lit_lights;
+  j.tree_cost = sc.bvh.sah_cost;
   j.layered = sc.dev.layered != 0;
   j.area = sc.dev.em_count > 0 || env != nullptr;
   j.wide = sc.dev.nodes4 ? j.req.wide_nodes & (uint32_t)(WIDE_EXTENSION | WIDE_SHADOW) : 0u;
@@ -284,17 +286,54 @@ pt_status ensure_wavefront(pt_context *ctx, uint32_t capacity, uint32_t shadow_s
   return PT_OK;
 }
 
-// Paths of a refine up to which the megakernel runs it, where nobody chose
-// the schedule. A wavefront wave is some seventy short launches whatever its
-// size; up to about one resident set of threads (148 SMs x 384) a path's own
-// chain of vertices is shorter. Device and wall time of one refine, 8 bounces,
-// wavefront / megakernel in ms: without area lights (sphere grid, material
-// extensions) 16 K paths 1.06 / 0.53 and 1.20 / 0.52, 64 K 1.28 / 0.71 and
-// 1.36 / 0.78, 131 K 1.41 / 1.15 and 1.34 / 1.25, 262 K 1.62 / 1.96 and 1.44 /
-// 2.12; with them (Cornell box, 100k soup: the f64 sampling is in its loop)
-// 4 K 0.74 / 0.37 and 2.55 / 2.43, 16 K 0.80 / 0.48 and 2.83 / 2.64, 32 K
-// 0.84 / 0.83 and 3.13 / 2.97, 64 K 0.87 / 1.21 and 3.30 / 4.68.
-constexpr uint64_t kSmallRefine = 96u << 10, kSmallRefineArea = 24u << 10;
+// Whether the megakernel runs a refine of one wave of `paths` paths where
+// nobody chose the schedule. A wavefront wave is some seventy short launches
+// whatever its size, each as long as its longest ray; the megakernel's time,
+// up to about one resident set of threads, is that of the longest path: its
+// vertices, and one after the other the shadow rays of each, over the
+// two-child nodes. So it wins where there are many vertices (every one saves
+// eight launches), few shadow rays a vertex and short walks. The walk's
+// length is the tree's SAH cost (a random ray's expected visits and tests),
+// not its triangle count: 17 for 200k triangles of spheres, 56 for the
+// heightfield and its spheres, 77 / 374 / 1,412 for soups of 10k / 100k /
+// 500k.
+//
+// Wall ms of one refine, wavefront / megakernel (without emitters; L lights):
+//   8 bounces, 16 K paths: spheres L1 1.16 / 0.47, L4 1.30 / 0.88, L8 1.40 /
+//     1.44; soup 10k L2 1.83 / 1.13, L4 1.95 / 1.71; soup 100k L1 2.57 / 1.71,
+//     L4 2.88 / 3.12; soup 500k L1 3.53 / 2.82, L2 at 4 K 3.21 / 3.34, L4 3.79
+//     / 4.54.
+//   2 bounces, 16 K: spheres L2 0.49 / 0.38, L4 0.51 / 0.56; soup 10k L1 0.62
+//     / 0.49, L4 0.67 / 0.88; soup 500k L1 1.17 / 1.17, at 256 paths 0.84 / 1.09.
+//   1 bounce, 16 K: spheres L1 0.31 / 0.24, L4 0.33 / 0.42.
+//   8 bounces, 48 / 64 / 96 K: spheres L1 1.30 / 0.56, 1.36 / 0.62, 1.41 /
+//     0.82; Cornell box without its emitter L4 0.78 / 0.80, 0.80 / 1.05, 0.85 /
+//     1.44; soup 500k L1 3.95 / 3.27, 4.05 / 4.56, 4.29 / 5.45.
+//   With area lights the f64 sampling is in the path's loop: Cornell box, 8
+//     bounces, 24 / 48 K: 0.81 / 0.61, 0.84 / 0.92.
+// Over 4,422 sizes, bounce counts, light counts and scenes of that kind no
+// refine that the rule takes was more than 8 % (11 us) slower than the
+// wavefront, and of 429 that it took among others drawn at random none more
+// than 5 % (half the time in the median). A rule by paths and area lights
+// alone took three of ten wrongly, at up to three times the wavefront's time.
+bool small_refine(const std::vector<Job> &jobs, uint64_t paths) {
+  uint32_t bounces = UINT32_MAX, shadow = 0;
+  double cost = 0.0;
+  bool area = false;
+  for (const Job &jb : jobs) {
+    bounces = std::min(bounces, jb.iterations - 1);
+    shadow = std::max(shadow, jb.lit_lights + (jb.area ? 1u : 0u));  // rays a vertex
+    cost = std::max(cost, std::isnan(jb.tree_cost) ? (double)INFINITY : jb.tree_cost);
+    area = area || jb.area;
+  }
+  // Most shadow rays a vertex by tree cost (below 64, below 128, above) and
+  // bounces (below 2, below 8, more); -1: none of the kind.
+  static const int most[3][3] = {{1, 2, 4}, {0, 1, 2}, {-1, -1, 1}};
+  const int c = cost < 64.0 ? 0 : (cost < 128.0 ? 1 : 2), v = bounces < 2 ? 0 : (bounces < 8 ? 1 : 2);
+  if ((int64_t)shadow > most[c][v]) return false;
+  const bool light = c == 0 && v == 2 && shadow <= 2;
+  return paths <= (area ? 24u << 10 : (light ? 64u << 10 : 48u << 10));
+}
 
 // Restores the context's schedule after a small refine.
 struct ScheduleScope {
@@ -343,11 +382,9 @@ pt_status run_jobs(pt_context *ctx, std::vector<pt_tracer *> &tracers, std::vect
     max_slots = std::max(max_slots, slots);
   }
   ScheduleScope scope{ctx, ctx->schedule};
-  if (ctx->schedule == PT_SCHEDULE_WAVEFRONT && !ctx->schedule_fixed && !ctx->stage_timing && waves.size() == 1) {
-    bool area = false;
-    for (const Job &jb : jobs) area = area || jb.area;
-    if (max_slots <= (area ? kSmallRefineArea : kSmallRefine)) ctx->schedule = PT_SCHEDULE_MEGAKERNEL;
-  }
+  if (ctx->schedule == PT_SCHEDULE_WAVEFRONT && !ctx->schedule_fixed && !ctx->stage_timing && waves.size() == 1 &&
+      small_refine(jobs, max_slots))
+    ctx->schedule = PT_SCHEDULE_MEGAKERNEL;
   // Overlapped waves need the wavefront, two or more waves, and no per-stage
   // timing (whose events sit on one stream).
   const bool overlap = ctx->overlap_waves && ctx->schedule == PT_SCHEDULE_WAVEFRONT && waves.size() >= 2 &&

@@ -146,6 +146,8 @@ struct Job {
   uint32_t iterations = 1;
   uint32_t shadow_slots = 1;
   uint32_t scene_key = 0;  // only orders the packing (locality)
+  uint32_t lit_lights = 0;  // SceneHost::lit_lights
+  double tree_cost = 0.0;  // the tree's SAH cost: a random ray's expected visits and tests
   bool layered = false;    // some triangle's material is not plain: the wave runs the layered shading too
   bool area = false;       // emissive triangles or an environment: the wave runs k_wf_nee
   uint32_t wide = 0;       // WIDE_* bits of the request that its scene's layouts honour

@@ -1348,6 +1348,8 @@ std::string build_scene_image(const pt_scene_desc &desc, SceneImage &img, bool w
     lights[j].l = desc.lights[j];
     lights[j].cos_outer = std::cos(desc.lights[j].outer_cone_angle);
     lights[j].cos_inner = std::cos(desc.lights[j].inner_cone_angle);
+    const pt_light &pl = desc.lights[j];
+    if (pl.intensity != 0.0f && (pl.color[0] != 0.0f || pl.color[1] != 0.0f || pl.color[2] != 0.0f)) ++img.lit_lights;
   }
 
   // EmissiveLights::build: the mean emitted radiance of each material, then
@@ -1728,6 +1730,7 @@ std::string commit_scene(const SceneImage &img, SceneHost &out, bool &oom, cudaS
   out.pool_texels = img.pool_bytes / sizeof(float4);
   out.bvh = img.bvh;
   out.light_count = img.light_count;
+  out.lit_lights = img.lit_lights;
   return "";
 }
 

@@ -108,6 +108,7 @@ struct SceneImage {
   uint64_t tri_count = 0;
   BvhBuildStats bvh;
   uint32_t light_count = 0;
+  uint32_t lit_lights = 0;  // of those, the ones with any radiance (the others send no shadow ray)
   // Host time of build_scene_image: total, tables (textures and their mips,
   // materials, lights, emissive tables), BVH build, the blob fill (corner
   // streams and tables copied into place).
@@ -123,6 +124,7 @@ struct SceneHost {
   uint64_t pool_texels = 0;  // texels of every mip chain (dev.texels)
   BvhBuildStats bvh;
   uint32_t light_count = 0;
+  uint32_t lit_lights = 0;  // of those, the ones with any radiance (the others send no shadow ray)
   bool device_bvh = false;  // the BVH was built on the GPU
   // Host wall time of upload_scene: host image, arena allocation + copy,
   // device BVH build, total.
