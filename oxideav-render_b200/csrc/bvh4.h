@@ -18,6 +18,19 @@
 
 namespace ptd {
 
+// The last plane of the grid origin + k * s on or below v, and the first on
+// or above it. The planes are exact in f64 (k is at most 2^8, origin and s
+// span fewer than 53 bits), v - origin need not be: a plane that its rounding
+// put on the wrong side of v moves by one.
+PT_HD double lower_plane(double v, double origin, double s) {
+  const double k = floor((v - origin) / s);
+  return origin + k * s > v ? k - 1.0 : k;
+}
+PT_HD double upper_plane(double v, double origin, double s) {
+  const double k = ceil((v - origin) / s);
+  return origin + k * s < v ? k + 1.0 : k;
+}
+
 // Fills `out` from the boxes of up to four children (lo[axis][child],
 // hi[axis][child]; used for refs other than kEmptyChild). Every stored plane
 // lies on or outside the box it stands for: the lower ones are rounded down
@@ -40,8 +53,8 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
     bool grid = range >= 0.0 && range < 1.0e38;
     if (grid) {
       frexp(range / 253.0, &e);
-      // Not finer than the coordinates can resolve: the f64 sums below stay
-      // exact, and a box without extent gets a grid all the same.
+      // Not finer than the coordinates can resolve: the planes stay exact in
+      // f64, and a box without extent gets a grid all the same.
       int least = -100;
       const double most = fmax(fabs((double)l), fabs((double)h));
       if (most > 0.0) {
@@ -58,9 +71,10 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
         grid = false;
         break;
       }
-      const double want = (double)l - wide;
-      float b = (float)want;
-      if ((double)b > want) b = nextafterf(b, -INFINITY);
+      // The first plane, base + wide: on or below l. Where l is tiny against
+      // the grid, l - wide rounds to -wide, which would place it at zero.
+      float b = (float)((double)l - wide);
+      while ((double)b + wide > (double)l) b = nextafterf(b, -INFINITY);
       if (!(fabsf(b) < 1.0e38f)) {
         grid = false;
         break;
@@ -68,7 +82,7 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
       origin = (double)b + wide;
       base[a] = b;
       step[a] = (float)wide;
-      if (ceil(((double)h - origin) / s) <= 255.0) break;
+      if (upper_plane((double)h, origin, s) <= 255.0) break;
     }
     qlo[a] = 0u;
     qhi[a] = 0u;
@@ -82,8 +96,8 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
         l8 = 0u;
         h8 = 255u;
         if (grid && lo[a][i] <= hi[a][i]) {
-          l8 = (uint32_t)fmax(floor(((double)lo[a][i] - origin) / s), 0.0);
-          h8 = (uint32_t)ceil(((double)hi[a][i] - origin) / s);
+          l8 = (uint32_t)lower_plane((double)lo[a][i], origin, s);
+          h8 = (uint32_t)upper_plane((double)hi[a][i], origin, s);
         }
       }
       qlo[a] |= l8 << (8 * i);

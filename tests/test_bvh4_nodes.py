@@ -52,13 +52,28 @@ def test_planes_enclose_the_boxes(size, offset, children):
                     assert pl > ph  # an unused slot is missed
                     continue
                 tl, th = Fraction(float(lo[c])), Fraction(float(hi[c]))
-                # The f64 rounding of the grid origin is below 2^-38 quanta.
-                assert pl <= tl + quantum / 2 ** 30 and ph >= th - quantum / 2 ** 30
+                assert pl <= tl and ph >= th
                 assert pl >= tl - 2 * quantum and ph <= th + 2 * quantum
             # Eight bits over the node's extent, plus what the rounding of the
             # base to f32 needs at this distance from zero.
             assert quantum <= max(Fraction(grid) / 63, Fraction(float(np.abs(a[ax]).max())) / 2 ** 22,
                                   Fraction(2) ** -99)
+
+
+# Bounds next to zero against the grid, whose distance from the grid's origin
+# f64 cannot hold: -1e-30 below an extent of 1, 1e-30 above one, and both
+# next to a plane inside.
+@pytest.mark.parametrize("lo,hi", [(-1e-30, 1.0), (-1.0, 1e-30), (-1e-30, 1e-30), (-1e-38, 3.0), (-7e4, 1e-20),
+                                   (-1e-45, 1e9), (1e-30, 2.0), (-3.0, -1e-30)])
+def test_planes_enclose_bounds_next_to_zero(lo, hi):
+    inner = np.float32((lo + hi) / 2)
+    a = np.array([[lo, lo, np.float32(-1e-30) if lo < -1e-30 < hi else lo, inner]] * 3, np.float32)
+    b = np.array([[hi, inner, hi, np.float32(1e-30) if inner < 1e-30 < hi else hi]] * 3, np.float32)
+    base, step, words = pack(a, b, [1, 2, 3, 4])
+    for ax in range(3):
+        for c in range(4):
+            (pl, ph), _ = planes(base, step, words, ax, c)
+            assert pl <= Fraction(float(a[ax, c])) and ph >= Fraction(float(b[ax, c])), (ax, c)
 
 
 @pytest.mark.parametrize("bad", [np.inf, np.nan, 3e38])
