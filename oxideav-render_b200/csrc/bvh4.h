@@ -18,16 +18,34 @@
 
 namespace ptd {
 
+// x = m * 2^e with m in [1/2, 1): e, for a normal x; and 2^e. A refit of a
+// small scene is one chain of nodes from a leaf to the root, whose length is
+// the latency of this file's arithmetic: no divisions and no library calls
+// (with them the device part of refitting a 4,616-triangle scene took 0.23 ms,
+// without 0.22, over full-precision nodes 0.20; larger scenes within noise).
+PT_HD int exponent_of(double x) {
+  uint64_t b;
+  memcpy(&b, &x, 8);
+  return (int)(b >> 52 & 0x7ffu) - 1022;
+}
+PT_HD double power_of_two(int e) {
+  const uint64_t b = (uint64_t)(e + 1023) << 52;
+  double x;
+  memcpy(&x, &b, 8);
+  return x;
+}
+
 // The last plane of the grid origin + k * s on or below v, and the first on
-// or above it. The planes are exact in f64 (k is at most 2^8, origin and s
+// or above it; s is a power of two and `inv` its reciprocal, so the product
+// is the quotient. The planes are exact in f64 (k is at most 2^8, origin and s
 // span fewer than 53 bits), v - origin need not be: a plane that its rounding
 // put on the wrong side of v moves by one.
-PT_HD double lower_plane(double v, double origin, double s) {
-  const double k = floor((v - origin) / s);
+PT_HD double lower_plane(double v, double origin, double s, double inv) {
+  const double k = floor((v - origin) * inv);
   return origin + k * s > v ? k - 1.0 : k;
 }
-PT_HD double upper_plane(double v, double origin, double s) {
-  const double k = ceil((v - origin) / s);
+PT_HD double upper_plane(double v, double origin, double s, double inv) {
+  const double k = ceil((v - origin) * inv);
   return origin + k * s < v ? k + 1.0 : k;
 }
 
@@ -48,24 +66,29 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
         l = fminf(l, lo[a][i]);
         h = fmaxf(h, hi[a][i]);
       }
-    int e = 0;
+    int e = -100;
     const double range = (double)h - (double)l;
     bool grid = range >= 0.0 && range < 1.0e38;
     if (grid) {
-      frexp(range / 253.0, &e);
+      // The extent in 126 to 253 quanta.
+      if (range > 0.0) {
+        e = exponent_of(range) - 8;
+        if (range >= 253.0 * power_of_two(e)) ++e;
+      }
       // Not finer than the coordinates can resolve: the planes stay exact in
       // f64, and a box without extent gets a grid all the same.
       int least = -100;
       const double most = fmax(fabs((double)l), fabs((double)h));
       if (most > 0.0) {
-        frexp(most, &least);
-        least = least - 30 < -100 ? -100 : least - 30;
+        least = exponent_of(most) - 30;
+        if (least < -100) least = -100;
       }
-      e = range == 0.0 || e < least ? least : e;
+      if (range == 0.0 || e < least) e = least;
     }
-    double s = 1.0, origin = 0.0;
+    double s = 1.0, inv = 1.0, origin = 0.0;
     for (; grid; ++e) {
-      s = ldexp(1.0, e);
+      s = power_of_two(e);
+      inv = power_of_two(-e);
       const double wide = s * 32768.0;
       if (!(wide < 1.0e38)) {
         grid = false;
@@ -82,7 +105,7 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
       origin = (double)b + wide;
       base[a] = b;
       step[a] = (float)wide;
-      if (upper_plane((double)h, origin, s) <= 255.0) break;
+      if (upper_plane((double)h, origin, s, inv) <= 255.0) break;
     }
     qlo[a] = 0u;
     qhi[a] = 0u;
@@ -96,8 +119,8 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
         l8 = 0u;
         h8 = 255u;
         if (grid && lo[a][i] <= hi[a][i]) {
-          l8 = (uint32_t)lower_plane((double)lo[a][i], origin, s);
-          h8 = (uint32_t)upper_plane((double)hi[a][i], origin, s);
+          l8 = (uint32_t)lower_plane((double)lo[a][i], origin, s, inv);
+          h8 = (uint32_t)upper_plane((double)hi[a][i], origin, s, inv);
         }
       }
       qlo[a] |= l8 << (8 * i);
