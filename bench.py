@@ -804,7 +804,12 @@ def stage_roofline(bc, peak, peak_kind, config_tag, wave_paths):
             "kernel": names[dom], "bytes_per_launch": stage_bytes[dom] / max(launches, 1),
             "ms_per_launch": stage[dom] / max(launches, 1), "launches": int(launches),
             "l2": profiled_l2(names[dom], config_tag, wave_paths),
-            "stage_share": stage[dom] / max(sum(v for v in stage.values() if v > 0), 1e-9)}
+            "stage_share": stage[dom] / max(sum(v for v in stage.values() if v > 0), 1e-9),
+            # What the profiles show the kernel waits for; "bound" names only
+            # the rate that "frac" is measured against.
+            "limited_by": {"extend": "instruction issue", "shadow": "instruction issue",
+                           "shade": "load latency and instruction fetch",
+                           "nee": "latency", "megakernel": "latency and instruction fetch"}.get(dom, "hbm")}
 
 
 def run_frame(ctx, api, torch, args, ws, rank, flush):

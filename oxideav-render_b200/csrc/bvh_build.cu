@@ -1119,8 +1119,8 @@ __global__ void k_sah_records(const float4 *plo, uint32_t n, const float *pos, c
 }
 
 // ---- small subtrees: nodes of at most kSahSmall triangles leave the level
-// rounds and are built whole by one thread each (the same split rule, an
-// in-place partition), in node ids reserved for them (2c - 2 per node of c
+// rounds and are built whole by a warp each (the same split rule, a stable
+// partition), in node ids reserved for them (2c - 2 per node of c
 // triangles; unused ids stay empty leaves that nothing references).
 constexpr uint32_t kSahSmall = 32;
 
@@ -1441,7 +1441,7 @@ std::string device_build_bvh_sah(SceneHost &sc, cudaStream_t st, uint32_t max_de
     n_deferred += nk - active;
     m = active;
   }
-  // Small subtrees, one thread each, in reserved node ids.
+  // Small subtrees, a warp each, in reserved node ids.
   if (n_deferred) {
     k_sah_small_reserve<<<grid_for(n_deferred), kThreads, 0, st>>>(deferred, n_deferred, nd, route);
     uint32_t *rt = scan_exclusive<uint32_t>(route, first_id, n_deferred, scan32, st);

@@ -829,9 +829,9 @@ pt_status launch_wave(pt_context *ctx, const DevRequest *d_reqs, const WaveSegme
     CK(ctx, cudaMemcpyAsync(w.desc, &wd, sizeof wd, cudaMemcpyHostToDevice, ws));
     const bool timed = timer && timer->events;
     if (ctx->use_graphs && !timed) {
-      // One captured graph per (bounce count, traversal variant, arena /
-      // whole wave, shade variant, material sort) replays the wave: one
-      // launch instead of ~6 per bounce.
+      // One captured graph per (bounce count, node layouts, claim chunk,
+      // traversal block size, arena / whole wave, shade variants, material
+      // sort) replays the wave: one launch instead of eight or nine a bounce.
       const uint32_t key = iters << 12 | w.all_wide << 10 | w.claim_chunk << 7 | (w.trav_threads == 128 ? 64u : 0u) |
                            (own_stream ? 4u * (1u + (uint32_t)arena) : 0u) | (w.shade_blocks == 4 ? 2u : 0u) |
                            (w.layered ? 32u : 0u) | w.sort_materials;

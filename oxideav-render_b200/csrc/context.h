@@ -33,14 +33,15 @@ struct pt_context {
   std::string err;
   std::map<uint32_t, std::unique_ptr<ptd::SceneHost>> scenes;
   uint32_t next_id = 1;
-  // The wavefront is the default schedule (C1: 646 M samples/s against
-  // about 200 M for the megakernel); pt_set_schedule / tuned choices change it.
+  // The wavefront is the default schedule (sphere grid at 512^2 and 256 spp:
+  // 1,064 M samples/s against 153 M for the megakernel); pt_set_schedule and
+  // tuned choices change it, small_refine does for one call.
   uint32_t schedule = PT_SCHEDULE_WAVEFRONT;
   // The schedule (or any setting of the wavefront) was chosen, by a call or
   // by the tuner: small refines keep it.
   bool schedule_fixed = false;
-  // Path slots per wave. 8 M measured best with overlapped waves (C1: 646 M
-  // samples/s against 613 M at 4 M and 474 M at 1 M, three in flight).
+  // Path slots per wave. 8 M measured best with overlapped waves (sphere grid:
+  // 1,062 M samples/s against 1,006 M at 4 M and 764 M at 1 M, three in flight).
   uint32_t wave_slots = 1u << 23;
   // WIDE_* bits: rays that walk the four-child node layout in the wavefront
   // (default: both kinds).
@@ -60,7 +61,8 @@ struct pt_context {
   static constexpr uint64_t kPoolKeep = 1ull << 30;
   ptd::HostStaging staging;  // pinned host image buffer of pt_scene_upload
   std::map<uint32_t, ptd::TuneChoice> tuned;  // by scene class (ptd::scene_class)
-  // Wavefront waves replayed as CUDA graphs (bounce count << 1 | sort -> exec).
+  // Wavefront waves replayed as CUDA graphs, by launch_wave's key: the bounce
+  // count and every choice that changes the launches.
   bool use_graphs = true;
   std::map<uint32_t, cudaGraphExec_t> graphs;
   float4 *d_out = nullptr;
@@ -94,8 +96,8 @@ struct pt_context {
   ptd::WaveBuffers wf_more[kMaxArenas - 1] = {};  // the others
   void *wf_arena_more[kMaxArenas - 1] = {};
   size_t wf_bytes_more[kMaxArenas - 1] = {};
-  // Waves in flight at once (0: one wave at a time). Three by default: C1
-  // +4 % over two, the soup and C2 within 1 % either way.
+  // Waves in flight at once (0: one wave at a time). Three by default: sphere
+  // grid 1,063 M samples/s, two 1,037 M, one 946 M; 500k soup 117, 117, 113 M.
   uint32_t overlap_arenas = 3;
   bool overlap_waves = true;    // overlap_arenas >= 2
   bool overlap_fixed = false;   // the count was set explicitly: tuned choices keep it

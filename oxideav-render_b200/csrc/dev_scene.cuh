@@ -149,10 +149,13 @@ PT_DEV int child_of(const int4 &c, uint32_t key) {
 }
 
 // Where the ray meets a node's grid on one axis: plane f = 1 + q / 32768
-// lies at t = step * f + near (or far), the offsets moved apart by the
-// rounding of (base - o) * inv (twice 2^-24 of it) and of the triangle
-// test's own translation by the origin, with room to spare: 2^-21 of a value
-// that is at least 32,768 quanta or the distance to the node.
+// lies at t = step * f + near (or far). The offsets are (base - o) * inv,
+// moved apart by 2^-21 of it: that covers the rounding of this product (twice
+// 2^-24 of it), which for an origin in or near the box is large against t
+// (32,768 quanta, so the slack is a 64th of one), and of the triangle test's
+// own translation by the origin. For an origin next to the base the offset
+// and its slack vanish; the planes then lie some 32,768 quanta away and all
+// rounding is relative to t, which child_key's widening covers.
 struct AxisPlanes {
   float step, off_near, off_far;
   uint32_t near_word, far_word;

@@ -32,8 +32,8 @@ namespace ptd {
 // Stack entries a thread keeps in shared memory. A node visit whose pushes
 // stay within them takes the short, branch-free way; L1 loses what they take.
 // Extend + shadow stage at 8 / 12 / 16 / 20 / 24 entries: 500k-triangle soup
-// 109.7 / 103.5 / 95.9 / 94.1 / 93.5 ms a frame, stress scene 69.1 / 64.5 /
-// 62.9 / 64.0 / 63.6 ms, sphere grid 49.5 / 48.7 / 48.6 / 49.1 / 49.2 ms.
+// 100.8 / 94.0 / 86.5 / 83.9 / 83.3 ms a frame, stress scene 62.0 / 56.6 /
+// 55.7 / 56.0 / 56.1 ms, sphere grid 50.6 / 49.5 / 49.3 / 49.7 / 49.6 ms.
 constexpr int kShortStack = 16;
 constexpr int kTravDone = (int)0x80000000;  // "no next node": neither a node index nor a leaf reference
 // Rows of a block's shared words, one word per thread each: the stack, then

@@ -9,10 +9,10 @@
 //                 estimation and the emission MIS pdf (the f64
 //                 spherical-triangle and environment sampling), kept out of
 //                 the shade kernel's instruction footprint;
-//   k_wf_shade    (wavefront_shade.cuh) emission, material, BSDF, NEE shadow-ray generation,
-//                 BSDF sampling, roulette; survivors are appended to the next
-//                 active queue and paths with shadow rays to the shadow queue
-//                 (warp-aggregated atomics);
+//   k_wf_shade    emission, material, BSDF, NEE shadow-ray generation, BSDF
+//                 sampling, roulette (wavefront_shade.cuh); survivors are
+//                 appended to the next active queue and paths with shadow
+//                 rays to the shadow queue (one atomic per block and queue);
 //   k_wf_shadow   one lane per queued shadow ray (ray k of every path
 //                 before ray k + 1): whether it reaches its light;
 //   k_wf_shadow_add  each path's visible contributions, added to its
@@ -163,10 +163,10 @@ __global__ void __launch_bounds__(256) k_wf_sort_scatter(WaveBuffers w, uint32_t
 // those shade would compute inline (the same functions on the same inputs).
 // 1,024 threads per SM (64 registers, a few spills): the sampling is latency
 // bound (CDF searches, dependent f64 steps), so occupancy beats the
-// spill-free 106-register form (Cornell box 1.95 ms a frame at 512 threads,
-// 1.74 at 768). The barrier keeps a block's warps on the same code, as in
-// k_wf_shade: blocks of 256 without it 1.73, with it 1.65, of 512 1.60
-// (stress scene 11.85 / 11.54 / 11.12).
+// spill-free 106-register form (Cornell box 2.06 ms a frame at 512 threads,
+// 1.81 at 768 of 80 registers). The barrier keeps a block's warps on the same
+// code, as in k_wf_shade: blocks of 256 without it 1.74, with it 1.66, of 512
+// 1.62 (stress scene 12.5 / 12.3 / 11.8).
 constexpr int kNeeThreads = 512, kNeeBlocks = 2;
 __global__ void __launch_bounds__(kNeeThreads, kNeeBlocks) k_wf_nee(WaveBuffers w, uint32_t iter) {
   if (!(w.desc->flags & WAVE_AREA_LIGHTS)) return;  // nothing to sample in this wave

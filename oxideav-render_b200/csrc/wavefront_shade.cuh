@@ -17,10 +17,11 @@ namespace ptd {
 // of scattered loads. A block's warps therefore start each vertex together
 // and fetch the same code (the barrier of the loop's condition), and the
 // plain materials' smaller code and state have a kernel of their own. Stage
-// times with neither / the barrier / both: sphere grid 27.1 / 26.4 / 21.4 ms
-// a frame, stress scene 47.7 / 31.3 / 29.0, material extensions 4.16 / 3.30 /
-// 2.90. Prefetching the next vertex's state made all of them slower (28.0 /
-// 52.7 / 4.2 without the barrier).
+// times with neither (and all of a path's state read and written) / the
+// barrier / both: sphere grid 31.0 / 27.4 / 20.2 ms a frame, stress scene
+// 46.9 / 27.3 / 25.1, material extensions 4.20 / 2.94 / 2.62. Prefetching the
+// next vertex's state made all of them slower (1 to 10 %, without the
+// barrier).
 template <int kThreads, int kBlocks, bool kPlain>
 __global__ void __launch_bounds__(kThreads, kBlocks) k_wf_shade(WaveBuffers w, uint32_t iter) {
   __shared__ BlockAppend<kThreads> append;

@@ -12,15 +12,15 @@ namespace ptd {
 // its lanes stand idle: it costs a few hundred instructions and a chain of
 // loads, which the whole warp waits for however few lanes take part. Extend
 // on the sphere grid / stress scene / 500k-triangle soup, ms a frame, at 10,
-// 14, 18 lanes: 26.5 / 37.8 / 56.2, 25.4 / 37.4 / 56.9, 24.7 / 36.8 / 58.6;
-// shadow rays, which are shorter: 24.1 / 26.0 / 38.9, 23.2 / 25.5 / 38.7,
-// 22.5 / 25.8 / 39.0. With every finished ray replaced at once, the first
-// form of these kernels took 33.4 / 52.7 / 92.3 against 30.8 / 48.5 / 85.3.
+// 14, 18 lanes: 27.4 / 33.5 / 50.9, 26.4 / 33.3 / 51.6, 25.9 / 32.7 / 53.3;
+// shadow rays, which are shorter: 24.1 / 22.6 / 34.5, 23.5 / 22.5 / 34.4,
+// 22.9 / 22.4 / 34.8. With every finished ray replaced at once 39.4 / 51.5 /
+// 72.1 and 35.6 / 27.2 / 53.4.
 constexpr int kRefillExtend = 14, kRefillShadow = 18;
 // Steps of one kind between votes (a vote and its control flow are a tenth
-// of a step): extend 25.2 / 37.1 / 56.5 with one node visit a vote, 23.6 /
-// 34.9 / 53.7 with two, 25.2 / 36.7 / 58.1 with three; with two triangle
-// tests as well 23.1 / 33.6 / 51.9.
+// of a step): extend 28.1 / 35.5 / 53.5 with one node visit a vote, 26.9 /
+// 34.0 / 52.5 with two, 27.0 / 33.7 / 52.9 with three; with two triangle
+// tests as well as two visits 26.4 / 33.3 / 51.6.
 constexpr int kStepsPerVote = 2;
 
 // The shared words of a traversal block: the stacks and counts by row (only
