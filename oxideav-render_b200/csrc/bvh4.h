@@ -18,11 +18,14 @@
 
 namespace ptd {
 
-// x = m * 2^e with m in [1/2, 1): e, for a normal x; and 2^e. A refit of a
-// small scene is one chain of nodes from a leaf to the root, whose length is
-// the latency of this file's arithmetic: no divisions and no library calls
-// (with them the device part of refitting a 4,616-triangle scene took 0.23 ms,
-// without 0.22, over full-precision nodes 0.20; larger scenes within noise).
+// Packing is on the path of every refit (a small scene's is one chain of
+// nodes from a leaf to the root) and of every host build: no divisions, no
+// library calls and few branches. Refit of a 4,616-triangle scene, device
+// part, with frexp, ldexp and 24 divisions a node / without: 0.23 / 0.22 ms
+// (full-precision nodes 0.20; larger scenes within noise); a host build's
+// time per node 205 / 129 ns.
+
+// x = m * 2^e with m in [1/2, 1): e, for a normal x; and 2^e.
 PT_HD int exponent_of(double x) {
   uint64_t b;
   memcpy(&b, &x, 8);
@@ -34,19 +37,29 @@ PT_HD double power_of_two(int e) {
   memcpy(&x, &b, 8);
   return x;
 }
+// The largest float at most x, for x zero or of a normal float's magnitude.
+PT_HD float float_below(double x) {
+  uint64_t b;
+  memcpy(&b, &x, 8);
+  b += (uint64_t)((int64_t)b >> 63) & 0x1fffffffu;  // magnitudes of negative values go up
+  b &= ~(uint64_t)0x1fffffffu;
+  memcpy(&x, &b, 8);
+  return (float)x;
+}
 
 // The last plane of the grid origin + k * s on or below v, and the first on
-// or above it; s is a power of two and `inv` its reciprocal, so the product
-// is the quotient. The planes are exact in f64 (k is at most 2^8, origin and s
-// span fewer than 53 bits), v - origin need not be: a plane that its rounding
-// put on the wrong side of v moves by one.
-PT_HD double lower_plane(double v, double origin, double s, double inv) {
-  const double k = floor((v - origin) * inv);
-  return origin + k * s > v ? k - 1.0 : k;
+// or above it, for v in [origin, origin + 2^30 s]; s is a power of two and
+// `inv` its reciprocal, so the product is the quotient. The planes are exact
+// in f64 (k is small, origin and s span fewer than 53 bits), v - origin need
+// not be: a plane that its rounding put on the wrong side of v moves by one.
+PT_HD int lower_plane(double v, double origin, double s, double inv) {
+  const int k = (int)((v - origin) * inv);
+  return k - (int)(origin + k * s > v);
 }
-PT_HD double upper_plane(double v, double origin, double s, double inv) {
-  const double k = ceil((v - origin) * inv);
-  return origin + k * s < v ? k + 1.0 : k;
+PT_HD int upper_plane(double v, double origin, double s, double inv) {
+  int k = (int)((v - origin) * inv);
+  k += (int)(origin + k * s < v);
+  return k + (int)(origin + k * s < v);
 }
 
 // Fills `out` from the boxes of up to four children (lo[axis][child],
@@ -63,8 +76,8 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
     float l = INFINITY, h = -INFINITY;
     for (int i = 0; i < 4; ++i)
       if (ref[i] != kEmptyChild) {
-        l = fminf(l, lo[a][i]);
-        h = fmaxf(h, hi[a][i]);
+        l = lo[a][i] < l ? lo[a][i] : l;  // NaN corners are passed over
+        h = hi[a][i] > h ? hi[a][i] : h;
       }
     int e = -100;
     const double range = (double)h - (double)l;
@@ -78,7 +91,7 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
       // Not finer than the coordinates can resolve: the planes stay exact in
       // f64, and a box without extent gets a grid all the same.
       int least = -100;
-      const double most = fmax(fabs((double)l), fabs((double)h));
+      const double most = -(double)l > (double)h ? -(double)l : (double)h;  // the larger magnitude, as l <= h
       if (most > 0.0) {
         least = exponent_of(most) - 30;
         if (least < -100) least = -100;
@@ -96,8 +109,8 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
       }
       // The first plane, base + wide: on or below l. Where l is tiny against
       // the grid, l - wide rounds to -wide, which would place it at zero.
-      float b = (float)((double)l - wide);
-      while ((double)b + wide > (double)l) b = nextafterf(b, -INFINITY);
+      float b = float_below((double)l - wide);
+      if ((double)b + wide > (double)l) b = nextafterf(b, -INFINITY);
       if (!(fabsf(b) < 1.0e38f)) {
         grid = false;
         break;
@@ -105,7 +118,7 @@ PT_HD void pack_bvh4(const float lo[3][4], const float hi[3][4], const int ref[4
       origin = (double)b + wide;
       base[a] = b;
       step[a] = (float)wide;
-      if (upper_plane((double)h, origin, s, inv) <= 255.0) break;
+      if (upper_plane((double)h, origin, s, inv) <= 255) break;
     }
     qlo[a] = 0u;
     qhi[a] = 0u;

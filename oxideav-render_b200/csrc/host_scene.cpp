@@ -1077,7 +1077,8 @@ void emit_tree(const std::vector<BNode> &in_nodes, const std::vector<uint32_t> &
           ch[best + 1] = nodes[opened].left + 1;
           ++nch;
         }
-        std::vector<Item> next;
+        Item next[4];
+        int nnext = 0;
         const BNode *cs[4] = {};
         int ref[4] = {kEmptyChild, kEmptyChild, kEmptyChild, kEmptyChild};
         for (int k = 0; k < nch; ++k) {
@@ -1088,11 +1089,11 @@ void emit_tree(const std::vector<BNode> &in_nodes, const std::vector<uint32_t> &
           } else {
             ref[k] = (int)out_nodes4.size();
             out_nodes4.push_back(Bvh4Node{});
-            next.push_back({ch[k], (uint32_t)ref[k]});
+            next[nnext++] = {ch[k], (uint32_t)ref[k]};
           }
         }
         out_nodes4[it.gpu] = pack(cs, ref);
-        for (auto r = next.rbegin(); r != next.rend(); ++r) st.push_back(*r);
+        while (nnext > 0) st.push_back(next[--nnext]);
       }
     }
   }
